@@ -28,8 +28,11 @@
 //   warps 2-5     : epilogue of the other accumulator, overlapping the next
 //                   tile's MMAs: tcgen05.ld of their 32 TMEM lanes, the
 //                   placement mask, a transpose through shared memory so that
-//                   each global store writes one row's 16 (or 32 tap-pair)
-//                   consecutive floats.
+//                   each global store writes one row's 16 consecutive floats
+//                   (or row pairs: value and difference to the next row, which
+//                   the warps read from one another's staged rows; the tiles
+//                   then step by 127 rows, the last row serving its
+//                   predecessor only).
 // Every mbarrier wait is bounded; on a timeout the CTA records an error,
 // drains what it issued, waits for its MMAs to retire and frees its TMEM.
 #include "ykb_internal.hpp"
@@ -158,11 +161,29 @@ __device__ __forceinline__ void step_of(int i, int kchunks, NearChunks nc, int& 
     }
 }
 
-static_assert((2 * kPairLead) % 4 == 0, "tap-pair rows start 16-byte aligned after the lead");
-constexpr int kEpiWarps = 4;
-constexpr int kEpiSplit = kEpiWarps / 4;             // epilogue warps per quarter of the TMEM lanes
+constexpr int kEpiWarps = 4;                          // one per quarter of the TMEM lanes
 constexpr int kFilterThreads = 64 + 32 * kEpiWarps;  // producer, MMA issuer, epilogue warps
-constexpr int kStagePitch = 19;                       // floats per staged row: 2 carried + 16 (odd: no bank conflicts)
+// floats per staged row of 16: 8-byte accesses of 16 lanes a row apart, and of
+// eight lanes along each of two rows, fall on distinct banks
+constexpr int kStagePitch = 18;
+// row pairs read the next row across warps: two buffers, one barrier a chunk
+constexpr int staging_floats(bool pair) { return (pair ? 2 : 1) * TM * kStagePitch; }
+// rows from one tile to the next
+constexpr int tile_rows(bool pair) { return pair ? TM - 1 : TM; }
+
+// all epilogue warps arrive; true when all of them passed true
+__device__ __forceinline__ bool epilogue_all(bool ok)
+{
+    uint32_t r;
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 p, %1, 0;\n"
+                 " barrier.cta.red.and.pred q, 1, %2, p;\n selp.u32 %0, 1, 0, q;\n}\n"
+                 : "=r"(r) : "r"(ok ? 1u : 0u), "n"(32 * kEpiWarps) : "memory");
+    return r != 0;
+}
+__device__ __forceinline__ void epilogue_sync()
+{
+    asm volatile("barrier.cta.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
+}
 
 // 16 consecutive TMEM columns of this warp's 32 lanes, one per register;
 // the registers are valid after tmem_wait_ld, which takes them as operands
@@ -212,7 +233,7 @@ __global__ void __launch_bounds__(kFilterThreads, 1) ramp_tc_kernel(
     unsigned char* a_ring = smem;
     unsigned char* b_ring = smem + STAGES * kAStageBytes;
     float* staging = reinterpret_cast<float*>(b_ring + STAGES * kBStageBytes);
-    uint64_t* full = reinterpret_cast<uint64_t*>(staging + kEpiWarps * 32 * kStagePitch);
+    uint64_t* full = reinterpret_cast<uint64_t*>(staging + staging_floats(PAIR));
     uint64_t* empty = full + STAGES;
     uint64_t* acc_full = empty + STAGES;
     uint64_t* acc_empty = acc_full + 2;
@@ -245,7 +266,7 @@ __global__ void __launch_bounds__(kFilterThreads, 1) ramp_tc_kernel(
             long it = 0, issued = 0;
             bool stop = false;
             for (long t = blockIdx.x; t < tiles && !stop; t += gridDim.x) {
-                const int m0 = static_cast<int>((t / col_tiles) * TM);
+                const int m0 = static_cast<int>((t / col_tiles) * tile_rows(PAIR));
                 const int n0 = static_cast<int>((t % col_tiles) * TN);
                 const NearChunks nc = near_chunks<TN>(n0, kchunks, near);
                 const int total = tile_steps<NSEG>(kchunks, nc);
@@ -313,20 +334,23 @@ __global__ void __launch_bounds__(kFilterThreads, 1) ramp_tc_kernel(
         __syncwarp();
     } else {
         // --------------------------------------------------- epilogue ---
-        // warp w reads TMEM lanes 32 (w % 4) ..: rows m0 + 32 (w % 4) + lane,
-        // columns [h TW, (h + 1) TW) of the tile, h = (w - 2) / 4.  Eight
-        // epilogue warps, or the next chunk's TMEM load issued before this
-        // one's stores, measured no faster: both take registers from the
+        // warp w reads TMEM lanes 32 (w % 4) ..: rows m0 + 32 (w % 4) + lane.
+        // Eight epilogue warps, or the next chunk's TMEM load issued before
+        // this one's stores, measured no faster: both take registers from the
         // preweight that runs beside this kernel
-        constexpr int TW = TN / kEpiSplit;
-        static_assert(TW % 16 == 0, "whole 16-column chunks per epilogue warp");
-        const int q = warp & 3, h = (warp - 2) >> 2;
-        float* stg = staging + (warp - 2) * 32 * kStagePitch;
+        const int q = warp & 3;
+        float* const mine = staging + (q * 32 + lane) * kStagePitch;  // this lane's staged row
+        const float* const rows0 = staging + q * 32 * kStagePitch;    // this warp's
         int tl = 0;
+        uint32_t buffer = 0;
         for (long t = blockIdx.x; t < tiles; t += gridDim.x, ++tl) {
             const int buf = tl & 1;
-            // the warp leaves together when a wait runs out
-            if (!__all_sync(0xffffffffu, bar_wait(&acc_full[buf], static_cast<uint32_t>(tl >> 1) & 1))) {
+            // the warp leaves together when a wait runs out; with row pairs,
+            // whose barriers span the epilogue warps, all of them do
+            bool ready = __all_sync(0xffffffffu,
+                bar_wait(&acc_full[buf], static_cast<uint32_t>(tl >> 1) & 1));
+            if constexpr (PAIR) ready = epilogue_all(ready);
+            if (!ready) {
                 if (lane == 0) {
                     atomicOr(err, kErrTimeout);
                     *(volatile int*)abort_flag = 1;
@@ -334,30 +358,30 @@ __global__ void __launch_bounds__(kFilterThreads, 1) ramp_tc_kernel(
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const long m0 = (t / col_tiles) * TM;
-            const int n0 = static_cast<int>((t % col_tiles) * TN) + h * TW;  // this warp's columns
+            const long m0 = (t / col_tiles) * tile_rows(PAIR);
+            const int n0 = static_cast<int>((t % col_tiles) * TN);
             const long wrow0 = m0 + q * 32;  // the warp's first row
             const long m = wrow0 + lane;
             // this lane's row keeps columns [lo, hi) (the samples placed in
             // the padded FFT row)
             int lo = 0, hi = 0;
+            // row pairs: the lane's row of the layout times four, with 2 for
+            // a view's first row and 1 for its last; -1 for a row that this
+            // tile does not write
+            int place = -1;
             if (m < rows) {
-                const FdkPreweightView& p = pwv[m / nv];
+                const int view = static_cast<int>(m / nv);
+                const FdkPreweightView& p = pwv[view];
                 lo = max(p.out_lo, 0);
                 hi = max(min(p.out_hi, nu), lo);
+                const int v = static_cast<int>(m - static_cast<long>(view) * nv);
+                if (q * 32 + lane < tile_rows(PAIR))
+                    place = static_cast<int>(m + view + 1) * 4 + (v == 0 ? 2 : 0) + (v == nv - 1 ? 1 : 0);
             }
-            // tap pairs: this warp writes the floats [X0, X1) of each row
-            // (float x holds f[(x + 1) >> 1]): from 2 n0 - 1, or -4 at
-            // column 0 (the pairs before the row are zero), up to the next
-            // warp's (or tile's) first float, or 2 nu (the right half of the
-            // last pair is zero)
-            const int X0 = n0 == 0 ? -4 : 2 * n0 - 1;
-            const int X1 = n0 + TW >= nu ? 2 * nu : 2 * (n0 + TW) - 1;
-            float carry0 = 0.f, carry1 = 0.f;  // columns c0 - 2 and c0 - 1 of the lane's row
             const uint32_t tcol = tmem + (static_cast<uint32_t>(q * 32) << 16) +
-                static_cast<uint32_t>(buf) * kAccCols + static_cast<uint32_t>(h * TW);
+                static_cast<uint32_t>(buf) * kAccCols;
 #pragma unroll 1
-            for (int c = 0; c < TW; c += 16) {
+            for (int c = 0; c < TN; c += 16) {
                 uint32_t r[16];
                 tmem_ld16(tcol + static_cast<uint32_t>(c), r);
                 tmem_wait_ld(r);
@@ -365,72 +389,55 @@ __global__ void __launch_bounds__(kFilterThreads, 1) ramp_tc_kernel(
                 float x[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) x[i] = __uint_as_float(r[i]);
-                // the next chunk's load runs while this one is stored
-
                 if (c0 < lo || c0 + 16 > hi) {
 #pragma unroll
                     for (int i = 0; i < 16; ++i)
                         if (static_cast<unsigned>(c0 + i - lo) >= static_cast<unsigned>(hi - lo)) x[i] = 0.f;
                 }
-                // staged row: columns c0 - 2 .. c0 + 15
-                float* srow = stg + lane * kStagePitch;
-                srow[0] = carry0;
-                srow[1] = carry1;
+                float* const srow = mine + (PAIR ? buffer : 0u);
+                const float* const staged = rows0 + (PAIR ? buffer : 0u);
 #pragma unroll
-                for (int i = 0; i < 16; ++i) srow[2 + i] = x[i];
-                carry0 = x[14];
-                carry1 = x[15];
-                __syncwarp();
+                for (int i = 0; i < 8; ++i)
+                    *reinterpret_cast<float2*>(srow + 2 * i) = make_float2(x[2 * i], x[2 * i + 1]);
                 // transposed: each store instruction writes whole row segments
                 if constexpr (PAIR) {
-                    if (vec) {
-                        // 16-byte blocks [xb, xb + 4), xb = 2 c0 - 4 + 4 t:
-                        // (f[m], f[m+1], f[m+1], f[m+2]), m = c0 - 2 + 2 t;
-                        // eight lanes a row, four rows a store
-                        const int t = lane & 7, g = lane >> 3;
-                        const int xb = 2 * c0 - 4 + 4 * t;
-                        const bool whole = xb >= X0 && xb + 4 <= X1;
-                        const bool some = xb + 4 > X0 && xb < X1;
+                    // the other buffer of the two is free for the next chunk: a
+                    // warp there has passed this chunk's barrier
+                    epilogue_sync();
+                    buffer ^= static_cast<uint32_t>(TM * kStagePitch);
+                    // a lane's 16 bytes: columns c0 + 2 t and + 1 of a row and
+                    // their differences to the next row; eight lanes a row,
+                    // four rows a store
+                    const int t8 = lane & 7, g = lane >> 3, u = c0 + 2 * t8;
 #pragma unroll
-                        for (int qq = 0; qq < 8; ++qq) {
-                            const int rr = 4 * qq + g;
-                            const long mr = wrow0 + rr;
-                            if (mr >= rows || !some) continue;
-                            const float* sp = stg + rr * kStagePitch + 2 * t;
-                            const float a = sp[0], b = sp[1], e = sp[2];
-                            float* dst = C + mr * 2 * ldc + 2 * kPairLead + xb;
-                            if (whole) {
-                                *reinterpret_cast<float4*>(dst) = make_float4(a, b, b, e);
-                            } else {
-                                if (xb >= X0 && xb < X1) dst[0] = a;
-                                if (xb + 1 >= X0 && xb + 1 < X1) dst[1] = b;
-                                if (xb + 2 >= X0 && xb + 2 < X1) dst[2] = b;
-                                if (xb + 3 >= X0 && xb + 3 < X1) dst[3] = e;
-                            }
-                        }
-                    } else {
-                        // lane l writes float 2 c0 - 1 + l, which is f[c0 + l / 2]
-                        const int xl = 2 * c0 - 1 + lane;
-                        for (int rr = 0; rr < 32; ++rr) {
-                            const long mr = wrow0 + rr;
-                            if (mr >= rows) break;
-                            float* dst = C + mr * 2 * ldc + 2 * kPairLead;
-                            if (xl >= X0 && xl < X1) dst[xl] = stg[rr * kStagePitch + 2 + (lane >> 1)];
-                            if (c0 == 0 && lane < 3) dst[-4 + lane] = 0.f;
-                        }
+                    for (int qq = 0; qq < 8; ++qq) {
+                        const int rr = 4 * qq + g;
+                        const int at = __shfl_sync(0xffffffffu, place, rr);
+                        if (at < 0 || u >= nu) continue;
+                        const float* sp = staged + rr * kStagePitch + 2 * t8;
+                        const float2 a = *reinterpret_cast<const float2*>(sp);
+                        float2 b = make_float2(0.f, 0.f);
+                        if (!(at & 1)) b = *reinterpret_cast<const float2*>(sp + kStagePitch);
+                        // the pitch ldc is even: the second column of the last
+                        // pair may lie in the padding, which no copy reads
+                        float4* dst = reinterpret_cast<float4*>(
+                            C + 2 * (static_cast<long>(at >> 2) * ldc + u));
+                        *dst = make_float4(a.x, b.x - a.x, a.y, b.y - a.y);
+                        if (at & 2) dst[-(ldc / 2)] = make_float4(0.f, a.x, 0.f, a.y);
                     }
                 } else {
-                    const int xe = min(n0 + TW, nu);  // this warp's columns [n0, xe)
+                    __syncwarp();
+                    const int xe = min(n0 + TN, nu);
                     if (vec) {
                         // 16-byte blocks: four lanes a row, eight rows a store
-                        const int t = lane & 3, g = lane >> 2;
-                        const int xb = c0 + 4 * t;
+                        const int t4 = lane & 3, g = lane >> 2;
+                        const int xb = c0 + 4 * t4;
 #pragma unroll
                         for (int qq = 0; qq < 4; ++qq) {
                             const int rr = 8 * qq + g;
                             const long mr = wrow0 + rr;
                             if (mr >= rows || xb >= xe) continue;
-                            const float* sp = stg + rr * kStagePitch + 2 + 4 * t;
+                            const float* sp = staged + rr * kStagePitch + 4 * t4;
                             float* dst = C + mr * ldc + xb;
                             if (xb + 4 <= xe) {
                                 *reinterpret_cast<float4*>(dst) = make_float4(sp[0], sp[1], sp[2], sp[3]);
@@ -444,23 +451,10 @@ __global__ void __launch_bounds__(kFilterThreads, 1) ramp_tc_kernel(
                         for (int rr = 0; rr < 32; rr += 2) {
                             const long mr = wrow0 + rr + half;
                             if (mr < rows && jj < xe)
-                                C[mr * ldc + jj] = stg[(rr + half) * kStagePitch + 2 + (lane & 15)];
+                                C[mr * ldc + jj] = staged[(rr + half) * kStagePitch + (lane & 15)];
                         }
                     }
-                }
-                __syncwarp();
-            }
-            if constexpr (PAIR) {
-                // the warp's last block, floats 2 (n0 + TW) - 4 .. - 1 =
-                // f[n0 + TW - 2], f[n0 + TW - 1] twice, f[n0 + TW]; the last
-                // is the next warp's, or zero when the columns end at nu
-                if (vec && m < rows) {
-                    const int xb = 2 * (n0 + TW) - 4;
-                    float* dst = C + m * 2 * ldc + 2 * kPairLead + xb;
-                    if (xb >= X0 && xb < X1) dst[0] = carry0;
-                    if (xb + 1 >= X0 && xb + 1 < X1) dst[1] = carry1;
-                    if (xb + 2 >= X0 && xb + 2 < X1) dst[2] = carry1;
-                    if (xb + 3 >= X0 && xb + 3 < X1) dst[3] = 0.f;
+                    __syncwarp();
                 }
             }
             // this accumulator is read out: the MMA warp may refill it
@@ -585,11 +579,12 @@ template <int TN, bool PAIR, int NSEG>
 cudaError_t launch_tn3(const CUtensorMap* a, const CUtensorMap* t, long rows, int nu, int nv,
     int kchunks, int near, const FdkPreweightView* pwv, float* C, int ldc, int* err, cudaStream_t s)
 {
-    // 16-byte stores need the rows 16-byte aligned: tap-pair rows are
-    // 2 ldc floats with kPairLead pairs before element 0
+    // 16-byte stores need the rows 16-byte aligned; row pairs always are (the
+    // plan's own buffers, even pitch)
     const int vec = reinterpret_cast<uintptr_t>(C) % 16 == 0 && ldc % (PAIR ? 2 : 4) == 0;
+    if (PAIR && !vec) return cudaErrorInvalidValue;
     const size_t smem = 1024 + STAGES * (kAStageBytes + TN * TK * 2) +
-        kEpiWarps * 32 * kStagePitch * sizeof(float) + (2 * STAGES + 5) * 8 + 16;
+        staging_floats(PAIR) * sizeof(float) + (2 * STAGES + 5) * 8 + 16;
     auto k = ramp_tc_kernel<TN, PAIR, NSEG>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
         static_cast<int>(smem));
@@ -599,7 +594,7 @@ cudaError_t launch_tn3(const CUtensorMap* a, const CUtensorMap* t, long rows, in
         (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess)
         return e;
     const int col_tiles = (nu + TN - 1) / TN;
-    const long tiles = static_cast<long>(col_tiles) * ((rows + TM - 1) / TM);
+    const long tiles = static_cast<long>(col_tiles) * ((rows + tile_rows(PAIR) - 1) / tile_rows(PAIR));
     const unsigned grid = static_cast<unsigned>(std::min<long>(tiles, sms));
     k<<<grid, kFilterThreads, smem, s>>>(a[0], a[1], a[2], t[0], t[1], t[2], rows, nu, nv,
         kchunks, near, col_tiles, tiles, pwv, C, ldc, vec, err);

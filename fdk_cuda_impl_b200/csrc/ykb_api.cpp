@@ -75,11 +75,18 @@ size_t volume_elems(const ykb_volume& v)
 // preweighted rows (4 as float or as two BF16 parts, 6 as three).
 int chunk_capacity(int n_views, int nu, int nv, int a_bytes)
 {
-    // preweighted rows + filtered tap pairs (8 B) per detector pixel
+    // preweighted rows + filtered row pairs (8 B) per detector pixel
     const size_t per_view = static_cast<size_t>(nu) * nv * (a_bytes + 8);
     const size_t budget = size_t(8) << 30;
     const size_t cap = std::max<size_t>(1, budget / std::max<size_t>(per_view, 1));
     return static_cast<int>(std::min<size_t>(n_views, cap));
+}
+
+// floats of one view's filtered rows in the plan's layout
+size_t filtered_view_floats(const ykb_fdk_plan* p)
+{
+    return p->layout == kFilteredPairs ? 2 * static_cast<size_t>(p->ld) * (p->nv + 1)
+                                       : static_cast<size_t>(p->ld) * p->nv;
 }
 
 } // namespace
@@ -189,7 +196,7 @@ YKB_API ykb_status ykb_fdk_plan_create_ex(const ykb_cone_view* views, int n_view
     if ((e = p->coef.alloc(sizeof(FdkViewCoef) * n_views)) != cudaSuccess ||
         (e = p->pwv.alloc(sizeof(FdkPreweightView) * n_views)) != cudaSuccess ||
         (e = p->ramp.alloc(sizeof(float) * hf.size())) != cudaSuccess ||
-        (e = p->err_flag.alloc(4 * sizeof(int))) != cudaSuccess ||
+        (e = p->err_flag.alloc(8 * sizeof(int))) != cudaSuccess ||
         (e = p->work_a.alloc(chunk_elems * a_bytes)) != cudaSuccess) {
         delete p;
         return cuda_status(e, "cudaMalloc (FDK plan workspace)");
@@ -200,7 +207,7 @@ YKB_API ykb_status ykb_fdk_plan_create_ex(const ykb_cone_view* views, int n_view
              cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaMemcpy(p->ramp.ptr, hf.data(), sizeof(float) * hf.size(),
              cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = cudaMemset(p->err_flag.ptr, 0, 4 * sizeof(int))) != cudaSuccess) {
+        (e = cudaMemset(p->err_flag.ptr, 0, 8 * sizeof(int))) != cudaSuccess) {
         delete p;
         return cuda_status(e, "cudaMemcpy (FDK plan tables)");
     }
@@ -252,26 +259,26 @@ YKB_API ykb_status ykb_fdk_plan_create_ex(const ykb_cone_view* views, int n_view
             return cuda_status(e, "cudaStreamCreate");
         }
         e = fdk_tma_box(p->coef.as<FdkViewCoef>(), n_views, make_grid(p->volume),
-            p->err_flag.as<int>() + 2, &p->tma_bw, &p->tma_bh, s);
+            p->err_flag.as<int>() + 4, &p->tma_box, s);
         cudaStreamDestroy(s);
         if (e != cudaSuccess) {
             delete p;
             return cuda_status(e, "backprojection box pre-pass");
         }
-        p->use_tma = p->tma_bw > 0 && fdk_tma_stages(p->tma_bw, p->tma_bh, kFilteredScalar) > 0;
+        p->use_tma = p->tma_box.row_w > 0;
     }
     // YKB_FDK_BP_PATH=rows|global selects the plain-row TMA or the global-load
     // backprojection instead of the default (tests compare the three paths)
     const char* path = std::getenv("YKB_FDK_BP_PATH");
     const bool force_rows = path && std::strcmp(path, "rows") == 0;
     if (path && std::strcmp(path, "global") == 0) p->use_tma = false;
-    // filtered workspace: tap pairs when their box fits the shared-memory
-    // ring, else plain rows; both with 16-byte row pitch (TMA)
-    p->layout = p->use_tma && !force_rows &&
-        fdk_tma_stages(p->tma_bw, p->tma_bh, kFilteredPairs) > 0 ? kFilteredPairs : kFilteredScalar;
-    p->ld = p->layout == kFilteredPairs ? (nu + kPairLead + 1) / 2 * 2 : (nu + 7) / 8 * 8;
-    const size_t filt_bytes = static_cast<size_t>(p->batch_capacity) * p->ld * nv *
-        (p->layout == kFilteredPairs ? 8 : 4);
+    // filtered workspace: row pairs when their box fits the shared-memory ring
+    // (the CUDA-core filter writes plain rows only), else plain rows; both with
+    // 16-byte row pitch (TMA)
+    p->layout = p->use_tma && !force_rows && p->tc_filter && p->tma_box.pair_w > 0
+        ? kFilteredPairs : kFilteredScalar;
+    p->ld = p->layout == kFilteredPairs ? (nu + 1) / 2 * 2 : (nu + 7) / 8 * 8;
+    const size_t filt_bytes = static_cast<size_t>(p->batch_capacity) * filtered_view_floats(p) * 4;
     if ((e = p->work_filtered.alloc(filt_bytes)) != cudaSuccess) {
         delete p;
         return cuda_status(e, "cudaMalloc (FDK filtered workspace)");
@@ -391,17 +398,17 @@ ykb_status filter_chunk_(ykb_fdk_plan* p, const void* proj, int proj_dtype, int 
             const __nv_bfloat16* const ac[3] = {a0 + row0 * p->lda, a0 + part + row0 * p->lda,
                 p->tc_parts == 3 ? a0 + 2 * part + row0 * p->lda : nullptr};
             if (nsub > 1) YKB_TRY_CUDA(cudaStreamWaitEvent(s, p->aux_done[b], 0));
-            const size_t out_row = layout == kFilteredPairs ? 2 * static_cast<size_t>(ldc)
-                                                            : static_cast<size_t>(ldc);
+            const size_t out_view = layout == kFilteredPairs
+                ? 2 * static_cast<size_t>(ldc) * (p->nv + 1) : static_cast<size_t>(ldc) * p->nv;
             YKB_TRY_CUDA(launch_fdk_ramp_tcgen05(ac, t, (v1 - v0) * p->nv, p->nu, p->lda, pwv + v0,
-                p->nv, dst + row0 * out_row, layout, ldc, p->tc_near, p->err_flag.as<int>(), s));
+                p->nv, dst + v0 * out_view, layout, ldc, p->tc_near, p->err_flag.as<int>(), s));
         }
         return YKB_OK;
     }
     YKB_TRY_CUDA(launch_fdk_preweight(proj, proj_dtype, pwv, parker, count, p->nu, p->nv,
         p->work_a.as<float>(), s));
     YKB_TRY_CUDA(launch_fdk_ramp_fp32(p->work_a.as<float>(), p->ramp.as<float>(), pwv, count,
-        p->nu, p->nv, dst, layout, ldc, s));
+        p->nu, p->nv, dst, ldc, s));
     return YKB_OK;
 }
 
@@ -430,14 +437,10 @@ ykb_status backproject_chunk_(ykb_fdk_plan* p, const void* filtered, int layout,
     }
     const FdkViewCoef* coef = p->coef.as<FdkViewCoef>() + first;
     const bool aligned = (reinterpret_cast<uintptr_t>(filtered) & 15) == 0;
-    if (layout == kFilteredPairs) {
+    if (layout == kFilteredPairs || (p->use_tma && ld % 4 == 0 && aligned)) {
         YKB_TRY_CUDA(launch_fdk_backproject_tma(static_cast<const float*>(filtered), layout, ld,
-            count, coef, count, p->nu, p->nv, grid, p->axial, p->tma_bw, p->tma_bh, vol,
-            accumulate, p->err_flag.as<int>(), s, nullptr, p->bp_wait));
-    } else if (p->use_tma && ld % 4 == 0 && aligned) {
-        YKB_TRY_CUDA(launch_fdk_backproject_tma(static_cast<const float*>(filtered), layout, ld,
-            count, coef, count, p->nu, p->nv, grid, p->axial, p->tma_bw, p->tma_bh, vol,
-            accumulate, p->err_flag.as<int>(), s, nullptr, p->bp_wait));
+            coef, count, p->nu, p->nv, grid, p->axial, p->tma_box, vol, accumulate,
+            p->err_flag.as<int>(), s, nullptr, p->bp_wait));
     } else {
         YKB_TRY_CUDA(launch_fdk_backproject(filtered, YKB_DTYPE_F32, coef, count, p->nu, p->nv,
             ld, grid, p->axial, vol, accumulate, s));
@@ -588,12 +591,12 @@ YKB_API ykb_status ykb_fdk_backproject(ykb_fdk_plan* p, const void* d_filtered,
     if (p->layout != kFilteredPairs)
         return backproject_chunk(p, d_filtered, kFilteredScalar, p->nu, view_offset, n_views,
             d_volume, clear_output ? 0 : 1, s);
-    // plain rows from the caller: re-laid as tap pairs in the plan workspace
+    // plain rows from the caller: re-laid as row pairs in the plan workspace
     const size_t view_elems = static_cast<size_t>(p->nu) * p->nv;
     for (int c = 0; c < n_views; c += p->batch_capacity) {
         const int cnt = std::min(p->batch_capacity, n_views - c);
         YKB_TRY_CUDA(launch_fdk_pairify(static_cast<const float*>(d_filtered) + c * view_elems,
-            p->nu, static_cast<long>(cnt) * p->nv, p->nu, p->work_filtered.as<float>(), p->ld, s));
+            p->nu, cnt, p->nu, p->nv, p->work_filtered.as<float>(), p->ld, s));
         const int accumulate = (c == 0 && clear_output) ? 0 : 1;
         if (const ykb_status st = backproject_chunk(p, p->work_filtered.ptr, kFilteredPairs, p->ld,
                 view_offset + c, cnt, d_volume, accumulate, s))
@@ -894,23 +897,23 @@ ykb_status prepare_pseudo(ykb_joseph_plan* p, cudaStream_t s)
     cudaError_t e;
     if ((e = p->fdk_coef.alloc(sizeof(FdkViewCoef) * coef.size())) != cudaSuccess ||
         (e = p->pseudo_coef.alloc(sizeof(PseudoViewCoef) * pc.size())) != cudaSuccess ||
-        (e = p->err_flag.alloc(4 * sizeof(int))) != cudaSuccess)
+        (e = p->err_flag.alloc(8 * sizeof(int))) != cudaSuccess)
         return cuda_status(e, "cudaMalloc (pseudo-matched tables)");
     YKB_TRY_CUDA(cudaMemcpyAsync(p->fdk_coef.ptr, coef.data(), p->fdk_coef.bytes,
         cudaMemcpyHostToDevice, s));
     YKB_TRY_CUDA(cudaMemcpyAsync(p->pseudo_coef.ptr, pc.data(), p->pseudo_coef.bytes,
         cudaMemcpyHostToDevice, s));
     YKB_TRY_CUDA(cudaMemsetAsync(p->err_flag.ptr, 0, p->err_flag.bytes, s));
-    p->pseudo_bw = p->pseudo_bh = 0;
+    p->pseudo_box = FdkTmaBox{};
     if (fdk_tma_available() && !std::getenv("YKB_PSEUDO_BP_GLOBAL")) {
-        int bw = 0, bh = 0;
+        FdkTmaBox box;
         YKB_TRY_CUDA(fdk_tma_box(p->fdk_coef.as<FdkViewCoef>(), p->n_views,
-            make_grid(p->volume), p->err_flag.as<int>() + 2, &bw, &bh, s));
-        if (bw > 0 && fdk_tma_stages(bw, bh, kFilteredPairs) > 0) {
-            const int ld = (p->nu + kPairLead + 1) / 2 * 2;
-            if (p->pairs.alloc(static_cast<size_t>(p->n_views) * p->nv * ld * 8) == cudaSuccess) {
-                p->pseudo_bw = bw;
-                p->pseudo_bh = bh;
+            make_grid(p->volume), p->err_flag.as<int>() + 4, &box, s));
+        if (box.pair_w > 0) {
+            const int ld = (p->nu + 1) / 2 * 2;
+            const size_t pair_floats = static_cast<size_t>(p->n_views) * (p->nv + 1) * ld * 2;
+            if (p->pairs.alloc(sizeof(float) * pair_floats) == cudaSuccess) {
+                p->pseudo_box = box;
                 p->pseudo_ld = ld;
             } else {
                 // without room for the staged pairs the bounds-checked kernel runs
@@ -928,14 +931,13 @@ ykb_status pseudo_bp(ykb_joseph_plan* p, const float* d_proj, float* d_volume, i
 {
     if (const ykb_status st = prepare_pseudo(p, s)) return st;
     const VolumeGrid g = make_grid(p->volume);
-    if (p->pseudo_bw > 0) {
-        YKB_TRY_CUDA(launch_fdk_pairify(d_proj, p->nu, static_cast<long>(p->n_views) * p->nv,
-            p->nu, p->pairs.as<float>(), p->pseudo_ld, s));
+    if (p->pseudo_box.pair_w > 0) {
+        YKB_TRY_CUDA(launch_fdk_pairify(d_proj, p->nu, p->n_views, p->nu, p->nv,
+            p->pairs.as<float>(), p->pseudo_ld, s));
         YKB_TRY_CUDA(launch_fdk_backproject_tma(p->pairs.as<float>(), kFilteredPairs,
-            p->pseudo_ld, p->n_views, p->fdk_coef.as<FdkViewCoef>(), p->n_views, p->nu, p->nv, g,
-            p->pseudo_axial, p->pseudo_bw, p->pseudo_bh, d_volume, accumulate,
-            p->err_flag.as<int>(), s,
-            p->pseudo_coef.as<PseudoViewCoef>()));
+            p->pseudo_ld, p->fdk_coef.as<FdkViewCoef>(), p->n_views, p->nu, p->nv, g,
+            p->pseudo_axial, p->pseudo_box, d_volume, accumulate, p->err_flag.as<int>(),
+            s, p->pseudo_coef.as<PseudoViewCoef>()));
         return YKB_OK;
     }
     YKB_TRY_CUDA(launch_pseudo_backproject(d_proj, p->fdk_coef.as<FdkViewCoef>(),

@@ -366,7 +366,7 @@ void build_pseudo_coefficients(const std::vector<FdkDerived>& g, const ykb_volum
         c.l2[4] = static_cast<float>(2.0 * ddot(d.detU, d.detV));
         c.l2[5] = static_cast<float>(ddot(d.detV, d.detV));
         c.k = std::fabs(d.plane) > 1e-12 ? static_cast<float>(cell / std::fabs(d.plane)) : 0.f;
-        c.ks = static_cast<float>(cell * std::fabs(d.plane));
+        c.kq = static_cast<float>(cell * d.plane * d.plane);
     }
 }
 

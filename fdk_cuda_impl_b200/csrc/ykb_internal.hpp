@@ -136,13 +136,13 @@ void build_ramp_kernel(int nu, double du, const ykb_filter& f,
 // YkFDKBpPrecompute.cu:104-122).
 // Since |P - S| = L den / SDD_plane for the detector point of P (den =
 // (P - S).n, n the unit detector normal), the weight equals
-// ks L / den^2 with ks = voxel volume |SDD_plane| / (du dv); the TMA
-// kernel uses that form, in which only L varies along an axial z-column.
+// kq |P - S| / den^3 with kq = voxel volume SDD_plane^2 / (du dv); the TMA
+// kernel uses that form, in which only |P - S| varies along an axial z-column.
 struct alignas(16) PseudoViewCoef {
     double src[4];
     float l2[6];  // l2[0] + u l2[1] + v l2[2] + u^2 l2[3] + u v l2[4] + v^2 l2[5]
     float k;
-    float ks;
+    float kq;
 };
 
 void build_pseudo_coefficients(const std::vector<FdkDerived>& g, const ykb_volume& vol,
@@ -176,14 +176,12 @@ struct VolumeGrid {
 VolumeGrid make_grid(const ykb_volume& v);
 
 // FDK
-// Layouts of filtered rows: plain floats [row][ld], or tap pairs
-// [row][ld] float2 where element kPairLead + u = (f[u], f[u+1]) for
-// u in [-kPairLead, nu) with f outside [0, nu) = 0.  The TMA
-// backprojection reads a row's two horizontal taps with one 8-byte load;
-// the two leading pairs keep the TMA box origin 16-byte aligned while
-// u = -1 still sees (0, f[0]).
+// Layouts of filtered rows: plain floats [view][nv][ld], or row pairs
+// [view][nv + 1][ld] float2 where element (n + 1, u) = (f[n][u],
+// f[n + 1][u] - f[n][u]) for n = -1 .. nv - 1, f zero outside the detector.
+// The TMA backprojection reads a voxel's four taps with two adjacent 8-byte
+// loads and lerps each column with one FMA.
 enum FilteredLayout : int { kFilteredScalar = 0, kFilteredPairs = 1 };
-constexpr int kPairLead = 2;
 // parker: per-(view, column) weights [n_views][nu] multiplied in after the
 // cosine weight (short scans), or nullptr
 cudaError_t launch_fdk_preweight(const void* proj, int proj_dtype,
@@ -191,7 +189,7 @@ cudaError_t launch_fdk_preweight(const void* proj, int proj_dtype,
     cudaStream_t s);
 cudaError_t launch_fdk_ramp_fp32(const float* pw_rows, const float* h_dev,
     const FdkPreweightView* pwv, int n_views, int nu, int nv, float* out,
-    int layout, int ldc, cudaStream_t s);
+    int ldc, cudaStream_t s);
 // BF16 split parts of the preweighted rows: parts[0], parts[1] and, when
 // parts[2] is not null, a third part (FP32-equivalent split)
 cudaError_t launch_fdk_preweight_split_bf16(const void* proj, int proj_dtype,
@@ -217,11 +215,12 @@ cudaError_t launch_fdk_backproject(const void* filtered, int dtype,
     cudaStream_t s);
 // TMA-staged backprojection (fdk_bp_tma.cu)
 bool fdk_tma_available();
-int fdk_tma_stages(int bw, int bh, int layout);
+// staged projection box as row pairs and as plain rows (width 0: not staged)
+struct FdkTmaBox { int pair_w = 0, pair_h = 0, row_w = 0, row_h = 0; };
 // z slices per tile of the TMA backprojection (slab work starts on a tile)
 int fdk_tma_z_tile();
 cudaError_t fdk_tma_box(const FdkViewCoef* coef, int n_views, const VolumeGrid& g,
-    int* scratch2, int* bw, int* bh, cudaStream_t s);
+    int* scratch3, FdkTmaBox* box, cudaStream_t s);
 // Limit of the TMA backprojection's pipeline waits (a wait that runs out
 // sets the error word and stops the CTA) and, for tests of that path, a view
 // whose copy the producer withholds (-1: none).  Waits that drain copies in
@@ -230,18 +229,19 @@ struct PipelineWait {
     unsigned long long limit_ns = 2000000000ull;
     int withheld_view = -1;
 };
-// pseudo != nullptr: the pseudo-matched weight of PseudoViewCoef replaces the
-// FDK depth weight (tap-pair layout only)
+// pseudo != nullptr: the pseudo-matched weight of PseudoViewCoef
+// replaces the FDK depth weight (row pairs only)
 cudaError_t launch_fdk_backproject_tma(const float* filtered, int layout, int ld,
-    int views_in_buffer, const FdkViewCoef* coef, int n_views, int nu, int nv,
-    const VolumeGrid& g, bool axial, int bw, int bh, float* vol, int accumulate, int* err,
-    cudaStream_t s, const PseudoViewCoef* pseudo = nullptr, PipelineWait pw = PipelineWait{});
+    const FdkViewCoef* coef, int n_views, int nu, int nv, const VolumeGrid& g, bool axial,
+    const FdkTmaBox& box, float* vol, int accumulate, int* err, cudaStream_t s,
+    const PseudoViewCoef* pseudo = nullptr, PipelineWait pw = PipelineWait{});
 // Pseudo-matched backprojection straight from projections [n][nv][nu] with
 // bounds-checked loads (used when the TMA box does not fit)
 cudaError_t launch_pseudo_backproject(const float* proj, const FdkViewCoef* coef,
     const PseudoViewCoef* pseudo, int n_views, int nu, int nv, const VolumeGrid& grid,
     float* vol, int accumulate, cudaStream_t s);
-cudaError_t launch_fdk_pairify(const float* in, int ld_in, long rows, int nu, float* out,
+// plain rows [views][nv][ld_in] -> row pairs [views][nv + 1][ldp]
+cudaError_t launch_fdk_pairify(const float* in, int ld_in, long views, int nu, int nv, float* out,
     int ldp, cudaStream_t s);
 
 // Joseph
@@ -308,7 +308,7 @@ struct ykb_fdk_plan {
     int layout = 0;              // FilteredLayout of the filtered workspace
     int lda = 0;                 // row pitch of the bf16 GEMM operands (tensor-core filter)
     bool use_tma = false;        // TMA-staged backprojection
-    int tma_bw = 0, tma_bh = 0;  // its projection box
+    ykb::FdkTmaBox tma_box;      // its projection box
     ykb::PipelineWait bp_wait;   // its pipeline-wait limit (tests shorten it)
     std::vector<ykb::FdkDerived> derived;
     ykb::DeviceBuffer coef;      // FdkViewCoef[n_views]
@@ -316,9 +316,9 @@ struct ykb_fdk_plan {
     ykb::DeviceBuffer ramp;      // float[2*nu-1]
     ykb::DeviceBuffer parker;    // float[n_views][nu] short-scan weights, or empty
     ykb::DeviceBuffer toeplitz_hi, toeplitz_lo, toeplitz_lo2;  // bf16 [nu][lda] split parts
-    ykb::DeviceBuffer work_a;    // preweighted rows: float, or the bf16 split parts in turn
+    ykb::DeviceBuffer work_a;    // preweighted rows : float, or the bf16 split parts in turn
     ykb::DeviceBuffer work_filtered;  // filtered projections (layout, pitch ld)
-    ykb::DeviceBuffer err_flag;  // int[4]: device error word, box pre-pass scratch
+    ykb::DeviceBuffer err_flag;  // int[8]: device error word, box pre-pass scratch
     // stage timing (ykb_fdk_stage_timing): a start and a stop event around
     // each filter (stage 0) and backprojection (stage 1) launch group, on the
     // stream that launches it; events are pooled and reused
@@ -375,12 +375,12 @@ struct ykb_joseph_plan {
     // pseudo-matched backprojection, set up on first use
     bool pseudo_ready = false;
     bool pseudo_axial = false;         // untilted detector: the axial column walk
-    int pseudo_bw = 0, pseudo_bh = 0;  // TMA projection box (0: bounds-checked loads)
-    int pseudo_ld = 0;                 // tap-pair row pitch
+    ykb::FdkTmaBox pseudo_box;         // TMA projection box (width 0: bounds-checked loads)
+    int pseudo_ld = 0;                 // row pitch of the row pairs
     ykb::DeviceBuffer fdk_coef;        // FdkViewCoef[n]
     ykb::DeviceBuffer pseudo_coef;     // PseudoViewCoef[n]
-    ykb::DeviceBuffer pairs;           // projections as tap pairs [n][nv][pseudo_ld]
-    ykb::DeviceBuffer err_flag;        // int[4]: device error word, box pre-pass scratch
+    ykb::DeviceBuffer pairs;           // projections as row pairs [n][nv + 1][pseudo_ld]
+    ykb::DeviceBuffer err_flag;        // int[8]: device error word, box pre-pass scratch
 };
 
 struct ykb_iter {

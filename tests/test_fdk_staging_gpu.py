@@ -1,0 +1,45 @@
+"""The staged backprojection's edges against the FP64 oracle: the row pairs of
+the filter epilogue across its 127-row tiles and views, and columns of tilted
+and untilted detectors over full, short and single z tiles.  Bound: the FP32
+form's 1e-5 (interpolation weights in FP32, sums of at most 48 views)."""
+import numpy as np
+import pytest
+
+from fdk_cuda_impl_b200.geometry import CircularScan, RampFilter, VolumeGrid
+from tests import cases as K
+
+pytestmark = pytest.mark.gpu
+FP32_TOL = 1e-5
+
+
+def _run(oracle, scan, grid, monkeypatch, **options):
+    import torch
+    from fdk_cuda_impl_b200.projectors import FdkPlan, JosephPlan
+    views, nu, nv = scan.views(), scan.channels, scan.rows
+    p = oracle.uniform((len(views), nv, nu), 0.5, 1.5, 4)
+    plan = FdkPlan(views, nu, nv, scan.scan_range, grid, RampFilter(), **options)
+    got = plan.execute(torch.from_numpy(p).cuda()).cpu().numpy()
+    plan.check()
+    plan.close()
+    vol = K.oracle_volume(oracle, grid)
+    ref = oracle.fdk(views, nu, nv, scan.scan_range, vol, oracle.filter_struct(1), p)
+    assert K.rel_rmse(got, ref) <= FP32_TOL
+    jp = JosephPlan(views, nu, nv, grid)
+    pseudo = jp.backproject_pseudo(torch.from_numpy(p).cuda()).cpu().numpy()
+    jp.check()
+    jp.close()
+    assert K.rel_rmse(pseudo, oracle.pseudo_bp(views, nu, nv, vol, p)) <= FP32_TOL
+
+
+@pytest.mark.parametrize("nu,nv", [(17, 1), (33, 2), (48, 126), (49, 127), (64, 128), (80, 129)])
+def test_row_pairs_across_filter_tiles(oracle, cuda_device, monkeypatch, nu, nv):
+    scan = CircularScan(7, 7, 500.0, 1000.0, nu, nv, 1.6, 1.6)
+    _run(oracle, scan, VolumeGrid(24, 20, 18, (1.0, 1.0, 1.0)), monkeypatch)
+
+
+@pytest.mark.parametrize("tilt", [(0.0, 0.0, 0.0), (0.006, -0.004, 0.008), (0.06, 0.05, -0.07)])
+@pytest.mark.parametrize("nz", [1, 33, 64, 69])
+def test_columns_over_z_tiles(oracle, cuda_device, monkeypatch, tilt, nz):
+    scan = CircularScan(20, 20, 400.0, 800.0, 64, 90, 1.7, 1.9, tilt_rad=tilt,
+                        offset_unv_mm=(0.8, 0.0, -1.1))
+    _run(oracle, scan, VolumeGrid(35, 33, nz, (1.1, 0.9, 1.2), (1.0, -0.5, 0.6)), monkeypatch)
