@@ -7,7 +7,8 @@
 //     512 threads keeps the 64 sums of a z column in registers over all views
 //     (the longer the column, the more voxels share the per-view column
 //     terms); a remainder of at most 32 slices runs as 32-voxel columns, the
-//     launch's last z layer;
+//     launch's last z layer.  A volume of few tiles also splits its views
+//     into jobs of their own (see split_count);
 //   * per view the detector box covering the tile's footprint is loaded with
 //     cp.async.bulk.tensor (3D tile mode, this GPU's memory only, no
 //     multicast) into a ring of shared-memory stages.  Out-of-detector
@@ -390,14 +391,16 @@ __device__ __forceinline__ BpSmem bp_smem(int BW, int BH, bool pair, int stages)
     return m;
 }
 
-// The launch's jobs, one per tile.  Tiles in order: layers of TX x TY tiles (x fastest), the
+// The launch's jobs: job j is tile j % n_tiles over the views of split
+// j / n_tiles.  Tiles in order: layers of TX x TY tiles (x fastest), the
 // ZT-slice layers from slice 0, then at most one layer of kZTail-slice tiles
 // (a short last part of the volume; it lies inside the ZT-slice layer of the
 // box pre-pass, so its footprints fit the same box).
 struct Schedule {
     int tiles_x, tiles_y, main_layers;
-    long n_jobs;
-    int n_views;
+    long n_tiles, n_jobs;
+    int n_views, splits;
+    long part_floats;  // distance of one split's sums from the next split's
 };
 
 // A walk over the (job, view) pairs of one CTA.
@@ -411,9 +414,10 @@ struct Cursor {
 __device__ __forceinline__ void cursor_open(Cursor& c, const Schedule& sc)
 {
     if (c.job >= sc.n_jobs) return;
-    const long t = c.job;
-    c.k = 0;
-    c.k1 = sc.n_views;
+    const int split = static_cast<int>(c.job / sc.n_tiles);
+    const long t = c.job - split * sc.n_tiles;
+    c.k = static_cast<int>(static_cast<long>(sc.n_views) * split / sc.splits);
+    c.k1 = static_cast<int>(static_cast<long>(sc.n_views) * (split + 1) / sc.splits);
     const long per_layer = static_cast<long>(sc.tiles_x) * sc.tiles_y;
     const int bz = static_cast<int>(t / per_layer);
     const int rem = static_cast<int>(t - bz * per_layer);
@@ -690,7 +694,7 @@ __device__ __forceinline__ bool bp_job(const BpSmem& sm, const CUtensorMap* map,
     if (bad) atomicOr(err, kErrFootprint);
     if (!active) return true;
     const long plane = static_cast<long>(g.nx) * g.ny;
-    float* dst = vol + static_cast<long>(y) * g.nx + x;
+    float* dst = vol + (cur.job / sc.n_tiles) * sc.part_floats + static_cast<long>(y) * g.nx + x;
 #pragma unroll
     for (int i = 0; i < ZC; ++i) {
         const int z = cur.za + i;
@@ -767,6 +771,30 @@ __global__ void __launch_bounds__(NTHREADS, 1) fdk_bp_tma_kernel(const __grid_co
     }
 }
 
+// out[i] (+)= the sum of the splits' parts, in order (HBM and L2 traffic; the
+// parts are `stride` floats apart, a multiple of 4; vec: out is 16-byte
+// aligned).
+__global__ void __launch_bounds__(256) sum_parts_kernel(const float* __restrict__ parts, int splits,
+    long stride, long n, int vec, float* __restrict__ out, int accumulate)
+{
+    const long step = static_cast<long>(gridDim.x) * blockDim.x;
+    const long first = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
+    const long n4 = vec ? n / 4 : 0;
+    for (long i = first; i < n4; i += step) {
+        float4 a = accumulate ? reinterpret_cast<const float4*>(out)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int s = 0; s < splits; ++s) {
+            const float4 b = __ldcs(reinterpret_cast<const float4*>(parts + s * stride) + i);
+            a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+        }
+        reinterpret_cast<float4*>(out)[i] = a;
+    }
+    for (long i = 4 * n4 + first; i < n; i += step) {
+        float a = accumulate ? out[i] : 0.f;
+        for (int s = 0; s < splits; ++s) a += __ldcs(parts + s * stride + i);
+        out[i] = a;
+    }
+}
+
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn()
 {
     static std::once_flag once;
@@ -815,9 +843,42 @@ Schedule tile_schedule(const VolumeGrid& g, int n_views)
     sc.main_layers = tail ? g.nz / ZT : (g.nz + ZT - 1) / ZT;
     sc.tiles_x = (g.nx + TX - 1) / TX;
     sc.tiles_y = (g.ny + TY - 1) / TY;
-    sc.n_jobs = static_cast<long>(sc.tiles_x) * sc.tiles_y * (sc.main_layers + (tail ? 1 : 0));
+    sc.n_tiles = static_cast<long>(sc.tiles_x) * sc.tiles_y * (sc.main_layers + (tail ? 1 : 0));
     sc.n_views = n_views;
+    sc.splits = 1;
+    sc.n_jobs = sc.n_tiles;
     return sc;
+}
+
+// floats of one split's sums: the volume's, to a multiple of four
+size_t part_stride(const VolumeGrid& g)
+{
+    return (static_cast<size_t>(g.nx) * g.ny * g.nz + 3) / 4 * 4;
+}
+
+// Splits of the views that finish a launch soonest: jobs run in rounds of one
+// per SM, a job takes its views plus about two views' time to fill the ring
+// and write its sums, and the splits' sums cost a launch (4 us) and a write and
+// a read (4 TB/s).  In units of a tile's view, 3 us.  64^3 x 60 views, 8 tiles:
+// 20 us in 18 splits, 171 in one; 128^3 x 180, 64 tiles: 257 and 503 us;
+// 256^3, 512 tiles, four rounds of 148 SMs for 3.5 rounds of work: 7 half
+// rounds; from about 20 rounds on, one split.
+int split_count(long n_tiles, int n_views, int sms, size_t floats, size_t part_floats)
+{
+    const long most = std::min<long>({static_cast<long>(part_floats / std::max<size_t>(floats, 1)),
+        static_cast<long>(n_views), 64L});
+    int best = 1;
+    double best_cost = 0.0;
+    for (int s = 1; s <= std::max(most, 1L); ++s) {
+        const double rounds = static_cast<double>((n_tiles * s + sms - 1) / sms);
+        double cost = rounds * ((n_views + s - 1) / s + 2.0);
+        if (s > 1) cost += (4e-6 + 4.0 * (2 * s + 2) * static_cast<double>(floats) / 4e12) / 3e-6;
+        if (s == 1 || cost < best_cost) {
+            best = s;
+            best_cost = cost;
+        }
+    }
+    return best;
 }
 
 cudaError_t sm_count(int* sms)
@@ -848,15 +909,27 @@ cudaError_t launch_form(const CUtensorMap& map, const FdkViewCoef* coef, const V
 
 template <bool AXIAL, bool PAIR, bool PSEUDO>
 cudaError_t launch_jobs(const CUtensorMap& map, const FdkViewCoef* coef, const VolumeGrid& g,
-    int bw, int bh, float* vol, int accumulate, int* err, const PseudoViewCoef* pseudo,
-    const Schedule& sc, PipelineWait pw, cudaStream_t s)
+    int bw, int bh, float* vol, int accumulate, int* err, const PseudoViewCoef* pseudo, float* parts,
+    size_t part_floats, Schedule sc, PipelineWait pw, cudaStream_t s)
 {
     int sms = 0;
-    const cudaError_t e = sm_count(&sms);
+    cudaError_t e = sm_count(&sms);
     if (e != cudaSuccess) return e;
-    return accumulate
-        ? launch_form<AXIAL, PAIR, PSEUDO, true>(map, coef, g, bw, bh, vol, err, pseudo, sc, sms, pw, s)
-        : launch_form<AXIAL, PAIR, PSEUDO, false>(map, coef, g, bw, bh, vol, err, pseudo, sc, sms, pw, s);
+    const size_t floats = part_stride(g);
+    sc.splits = split_count(sc.n_tiles, sc.n_views, sms, floats, parts ? part_floats : 0);
+    sc.n_jobs = sc.n_tiles * sc.splits;
+    if (sc.splits == 1)
+        return accumulate
+            ? launch_form<AXIAL, PAIR, PSEUDO, true>(map, coef, g, bw, bh, vol, err, pseudo, sc, sms, pw, s)
+            : launch_form<AXIAL, PAIR, PSEUDO, false>(map, coef, g, bw, bh, vol, err, pseudo, sc, sms, pw, s);
+    sc.part_floats = static_cast<long>(floats);
+    e = launch_form<AXIAL, PAIR, PSEUDO, false>(map, coef, g, bw, bh, parts, err, pseudo, sc, sms, pw, s);
+    if (e != cudaSuccess) return e;
+    const int vec = reinterpret_cast<uintptr_t>(vol) % 16 == 0;
+    const long n = static_cast<long>(g.nx) * g.ny * g.nz;
+    sum_parts_kernel<<<static_cast<unsigned>(std::min<long>((floats / 4 + 255) / 256, sms * 8)), 256, 0, s>>>(
+        parts, sc.splits, sc.part_floats, n, vec, vol, accumulate);
+    return cudaGetLastError();
 }
 
 } // namespace
@@ -891,10 +964,20 @@ int fdk_tma_z_tile() { return ZT; }
 
 bool fdk_tma_available() { return encode_fn() != nullptr; }
 
+size_t fdk_tma_part_floats(const VolumeGrid& g, int n_views)
+{
+    int sms = 0;
+    if (sm_count(&sms) != cudaSuccess) return 0;
+    const size_t floats = part_stride(g);
+    const int splits = split_count(tile_schedule(g, n_views).n_tiles, n_views, sms, floats,
+        (size_t(256) << 20) / sizeof(float));
+    return splits > 1 ? floats * splits : 0;
+}
+
 cudaError_t launch_fdk_backproject_tma(const float* filtered, int layout, int ld,
     const FdkViewCoef* coef, int n_views, int nu, int nv, const VolumeGrid& g, bool axial,
-    const FdkTmaBox& box, float* vol, int accumulate, int* err, cudaStream_t s,
-    const PseudoViewCoef* pseudo, PipelineWait pw)
+    const FdkTmaBox& box, float* vol, int accumulate, int* err, float* parts, size_t part_floats,
+    cudaStream_t s, const PseudoViewCoef* pseudo, PipelineWait pw)
 {
     auto enc = encode_fn();
     if (!enc) return cudaErrorNotSupported;
@@ -920,7 +1003,7 @@ cudaError_t launch_fdk_backproject_tma(const float* filtered, int layout, int ld
     const auto launch = pseudo ? (axial ? launch_jobs<true, true, true> : launch_jobs<false, true, true>)
         : pair ? (axial ? launch_jobs<true, true, false> : launch_jobs<false, true, false>)
                : (axial ? launch_jobs<true, false, false> : launch_jobs<false, false, false>);
-    return launch(map, coef, g, bw, bh, vol, accumulate, err, pseudo, sc, pw, s);
+    return launch(map, coef, g, bw, bh, vol, accumulate, err, pseudo, parts, part_floats, sc, pw, s);
 }
 
 // Plain rows [views][nv][ld_in] -> row pairs [views][nv + 1][ldp], the layout

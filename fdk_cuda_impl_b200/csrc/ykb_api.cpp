@@ -190,14 +190,17 @@ YKB_API ykb_status ykb_fdk_plan_create_ex(const ykb_cone_view* views, int n_view
     p->lda = p->tc_filter ? tc_filter_lda(nu) : nu;
     const int a_bytes = p->tc_parts == 3 ? 6 : 4;
     p->batch_capacity = chunk_capacity(n_views, nu, nv, a_bytes);
-    // work_a holds the preweighted rows: float, or the bf16 parts in turn
+    // work_a holds the preweighted rows: float, or the bf16 parts in turn; the
+    // backprojection, which runs after them in stream order, keeps the sums of
+    // split views there
     const size_t chunk_elems = static_cast<size_t>(p->batch_capacity) * p->lda * nv;
+    const size_t part_floats = fdk_tma_part_floats(make_grid(p->volume), n_views);
     cudaError_t e;
     if ((e = p->coef.alloc(sizeof(FdkViewCoef) * n_views)) != cudaSuccess ||
         (e = p->pwv.alloc(sizeof(FdkPreweightView) * n_views)) != cudaSuccess ||
         (e = p->ramp.alloc(sizeof(float) * hf.size())) != cudaSuccess ||
         (e = p->err_flag.alloc(8 * sizeof(int))) != cudaSuccess ||
-        (e = p->work_a.alloc(chunk_elems * a_bytes)) != cudaSuccess) {
+        (e = p->work_a.alloc(std::max(chunk_elems * a_bytes, part_floats * sizeof(float)))) != cudaSuccess) {
         delete p;
         return cuda_status(e, "cudaMalloc (FDK plan workspace)");
     }
@@ -440,7 +443,8 @@ ykb_status backproject_chunk_(ykb_fdk_plan* p, const void* filtered, int layout,
     if (layout == kFilteredPairs || (p->use_tma && ld % 4 == 0 && aligned)) {
         YKB_TRY_CUDA(launch_fdk_backproject_tma(static_cast<const float*>(filtered), layout, ld,
             coef, count, p->nu, p->nv, grid, p->axial, p->tma_box, vol, accumulate,
-            p->err_flag.as<int>(), s, nullptr, p->bp_wait));
+            p->err_flag.as<int>(), p->work_a.as<float>(), p->work_a.bytes / sizeof(float), s,
+            nullptr, p->bp_wait));
     } else {
         YKB_TRY_CUDA(launch_fdk_backproject(filtered, YKB_DTYPE_F32, coef, count, p->nu, p->nv,
             ld, grid, p->axial, vol, accumulate, s));
@@ -911,10 +915,13 @@ ykb_status prepare_pseudo(ykb_joseph_plan* p, cudaStream_t s)
             make_grid(p->volume), p->err_flag.as<int>() + 4, &box, s));
         if (box.pair_w > 0) {
             const int ld = (p->nu + 1) / 2 * 2;
+            const size_t part_floats = fdk_tma_part_floats(make_grid(p->volume), p->n_views);
             const size_t pair_floats = static_cast<size_t>(p->n_views) * (p->nv + 1) * ld * 2;
-            if (p->pairs.alloc(sizeof(float) * pair_floats) == cudaSuccess) {
+            if (p->pairs.alloc(sizeof(float) * (pair_floats + part_floats)) == cudaSuccess) {
                 p->pseudo_box = box;
                 p->pseudo_ld = ld;
+                p->pseudo_parts = p->pairs.as<float>() + pair_floats;
+                p->pseudo_part_floats = part_floats;
             } else {
                 // without room for the staged pairs the bounds-checked kernel runs
                 cudaGetLastError();
@@ -937,7 +944,7 @@ ykb_status pseudo_bp(ykb_joseph_plan* p, const float* d_proj, float* d_volume, i
         YKB_TRY_CUDA(launch_fdk_backproject_tma(p->pairs.as<float>(), kFilteredPairs,
             p->pseudo_ld, p->fdk_coef.as<FdkViewCoef>(), p->n_views, p->nu, p->nv, g,
             p->pseudo_axial, p->pseudo_box, d_volume, accumulate, p->err_flag.as<int>(),
-            s, p->pseudo_coef.as<PseudoViewCoef>()));
+            p->pseudo_parts, p->pseudo_part_floats, s, p->pseudo_coef.as<PseudoViewCoef>()));
         return YKB_OK;
     }
     YKB_TRY_CUDA(launch_pseudo_backproject(d_proj, p->fdk_coef.as<FdkViewCoef>(),

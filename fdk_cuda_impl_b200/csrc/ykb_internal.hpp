@@ -221,6 +221,9 @@ struct FdkTmaBox { int pair_w = 0, pair_h = 0, row_w = 0, row_h = 0; };
 int fdk_tma_z_tile();
 cudaError_t fdk_tma_box(const FdkViewCoef* coef, int n_views, const VolumeGrid& g,
     int* scratch3, FdkTmaBox* box, cudaStream_t s);
+// floats of workspace for the sums of split views (0: the volume has tiles
+// enough to fill the GPU)
+size_t fdk_tma_part_floats(const VolumeGrid& g, int n_views);
 // Limit of the TMA backprojection's pipeline waits (a wait that runs out
 // sets the error word and stops the CTA) and, for tests of that path, a view
 // whose copy the producer withholds (-1: none).  Waits that drain copies in
@@ -229,12 +232,13 @@ struct PipelineWait {
     unsigned long long limit_ns = 2000000000ull;
     int withheld_view = -1;
 };
-// pseudo != nullptr: the pseudo-matched weight of PseudoViewCoef
+// parts: workspace of part_floats floats for the sums of split views, or
+// nullptr.  pseudo != nullptr: the pseudo-matched weight of PseudoViewCoef
 // replaces the FDK depth weight (row pairs only)
 cudaError_t launch_fdk_backproject_tma(const float* filtered, int layout, int ld,
     const FdkViewCoef* coef, int n_views, int nu, int nv, const VolumeGrid& g, bool axial,
-    const FdkTmaBox& box, float* vol, int accumulate, int* err, cudaStream_t s,
-    const PseudoViewCoef* pseudo = nullptr, PipelineWait pw = PipelineWait{});
+    const FdkTmaBox& box, float* vol, int accumulate, int* err, float* parts, size_t part_floats,
+    cudaStream_t s, const PseudoViewCoef* pseudo = nullptr, PipelineWait pw = PipelineWait{});
 // Pseudo-matched backprojection straight from projections [n][nv][nu] with
 // bounds-checked loads (used when the TMA box does not fit)
 cudaError_t launch_pseudo_backproject(const float* proj, const FdkViewCoef* coef,
@@ -316,7 +320,7 @@ struct ykb_fdk_plan {
     ykb::DeviceBuffer ramp;      // float[2*nu-1]
     ykb::DeviceBuffer parker;    // float[n_views][nu] short-scan weights, or empty
     ykb::DeviceBuffer toeplitz_hi, toeplitz_lo, toeplitz_lo2;  // bf16 [nu][lda] split parts
-    ykb::DeviceBuffer work_a;    // preweighted rows : float, or the bf16 split parts in turn
+    ykb::DeviceBuffer work_a;    // preweighted rows (float, or the bf16 split parts in turn), then sums of split views
     ykb::DeviceBuffer work_filtered;  // filtered projections (layout, pitch ld)
     ykb::DeviceBuffer err_flag;  // int[8]: device error word, box pre-pass scratch
     // stage timing (ykb_fdk_stage_timing): a start and a stop event around
@@ -379,7 +383,9 @@ struct ykb_joseph_plan {
     int pseudo_ld = 0;                 // row pitch of the row pairs
     ykb::DeviceBuffer fdk_coef;        // FdkViewCoef[n]
     ykb::DeviceBuffer pseudo_coef;     // PseudoViewCoef[n]
-    ykb::DeviceBuffer pairs;           // projections as row pairs [n][nv + 1][pseudo_ld]
+    ykb::DeviceBuffer pairs;           // projections as row pairs [n][nv + 1][pseudo_ld], then
+    float* pseudo_parts = nullptr;     // the sums of split views
+    size_t pseudo_part_floats = 0;
     ykb::DeviceBuffer err_flag;        // int[8]: device error word, box pre-pass scratch
 };
 

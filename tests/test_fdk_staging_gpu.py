@@ -43,3 +43,34 @@ def test_columns_over_z_tiles(oracle, cuda_device, monkeypatch, tilt, nz):
     scan = CircularScan(20, 20, 400.0, 800.0, 64, 90, 1.7, 1.9, tilt_rad=tilt,
                         offset_unv_mm=(0.8, 0.0, -1.1))
     _run(oracle, scan, VolumeGrid(35, 33, nz, (1.1, 0.9, 1.2), (1.0, -0.5, 0.6)), monkeypatch)
+
+
+@pytest.mark.parametrize("tilt", [(0.0, 0.0, 0.0), (0.006, -0.004, 0.008)])
+@pytest.mark.parametrize("n,nz,views", [(16, 1, 3), (31, 21, 48), (64, 33, 90), (96, 130, 24)])
+def test_split_views_match_one_job_a_tile(oracle, cuda_device, monkeypatch, n, nz, views, tilt):
+    # volumes of few tiles split their views into jobs whose sums are added
+    # afterwards; the bounds-checked kernel (YKB_FDK_BP_PATH=global) sums every
+    # view in one thread from detector coordinates that it rounds to FP32: up
+    # to 7.6e-6 px (below 128 px) on white-noise rows, 1e-5 of their size.
+    # Also adding to a volume 4 bytes off a 16-byte boundary
+    import torch
+    from fdk_cuda_impl_b200.projectors import FdkPlan
+    scan = CircularScan(views, views, 400.0, 800.0, 70, 90, 3.0 * n / 64, 3.0 * n / 64, tilt_rad=tilt)
+    grid = VolumeGrid(n, n + 1, nz, (1.0, 1.0, 1.0))
+    p = torch.from_numpy(oracle.uniform((views, 90, 70), 0.5, 1.5, 5)).cuda()
+    split = FdkPlan(scan.views(), 70, 90, scan.scan_range, grid, RampFilter())
+    monkeypatch.setenv("YKB_FDK_BP_PATH", "global")
+    one = FdkPlan(scan.views(), 70, 90, scan.scan_range, grid, RampFilter())
+    a, b = split.execute(p), one.execute(p)
+    assert K.rel_rmse(a.cpu().numpy(), b.cpu().numpy()) <= 2e-5
+    assert torch.equal(a, split.execute(p))
+    flat = torch.full((a.numel() + 1,), 2.0, device="cuda")
+    shifted = flat[1:].view(a.shape)
+    shifted.copy_(b)
+    split.execute(p[:views // 2], shifted, clear=False)
+    split.execute(p[views // 2:], shifted, view_offset=views // 2, clear=False)
+    split.check()
+    assert flat[0].item() == 2.0
+    assert K.rel_rmse(shifted.cpu().numpy(), 2.0 * b.cpu().numpy()) <= 2e-5
+    split.close()
+    one.close()
