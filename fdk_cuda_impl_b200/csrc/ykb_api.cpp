@@ -190,17 +190,14 @@ YKB_API ykb_status ykb_fdk_plan_create_ex(const ykb_cone_view* views, int n_view
     p->lda = p->tc_filter ? tc_filter_lda(nu) : nu;
     const int a_bytes = p->tc_parts == 3 ? 6 : 4;
     p->batch_capacity = chunk_capacity(n_views, nu, nv, a_bytes);
-    // work_a holds the preweighted rows: float, or the bf16 parts in turn; the
-    // backprojection, which runs after them in stream order, keeps the sums of
-    // split views there
+    // work_a holds the preweighted rows: float, or the bf16 parts in turn
     const size_t chunk_elems = static_cast<size_t>(p->batch_capacity) * p->lda * nv;
-    const size_t part_floats = fdk_tma_part_floats(make_grid(p->volume), n_views);
     cudaError_t e;
     if ((e = p->coef.alloc(sizeof(FdkViewCoef) * n_views)) != cudaSuccess ||
         (e = p->pwv.alloc(sizeof(FdkPreweightView) * n_views)) != cudaSuccess ||
         (e = p->ramp.alloc(sizeof(float) * hf.size())) != cudaSuccess ||
         (e = p->err_flag.alloc(8 * sizeof(int))) != cudaSuccess ||
-        (e = p->work_a.alloc(std::max(chunk_elems * a_bytes, part_floats * sizeof(float)))) != cudaSuccess) {
+        (e = p->work_a.alloc(chunk_elems * a_bytes)) != cudaSuccess) {
         delete p;
         return cuda_status(e, "cudaMalloc (FDK plan workspace)");
     }
@@ -281,8 +278,11 @@ YKB_API ykb_status ykb_fdk_plan_create_ex(const ykb_cone_view* views, int n_view
     p->layout = p->use_tma && !force_rows && p->tc_filter && p->tma_box.pair_w > 0
         ? kFilteredPairs : kFilteredScalar;
     p->ld = p->layout == kFilteredPairs ? (nu + 1) / 2 * 2 : (nu + 7) / 8 * 8;
-    const size_t filt_bytes = static_cast<size_t>(p->batch_capacity) * filtered_view_floats(p) * 4;
-    if ((e = p->work_filtered.alloc(filt_bytes)) != cudaSuccess) {
+    // behind the row pairs, the sums of split views: the backprojection shares no
+    // workspace with the filter that it did not read before
+    p->filtered_floats = static_cast<size_t>(p->batch_capacity) * filtered_view_floats(p);
+    p->part_floats = p->layout == kFilteredPairs ? fdk_tma_part_floats(make_grid(p->volume), n_views) : 0;
+    if ((e = p->work_filtered.alloc(sizeof(float) * (p->filtered_floats + p->part_floats))) != cudaSuccess) {
         delete p;
         return cuda_status(e, "cudaMalloc (FDK filtered workspace)");
     }
@@ -443,7 +443,7 @@ ykb_status backproject_chunk_(ykb_fdk_plan* p, const void* filtered, int layout,
     if (layout == kFilteredPairs || (p->use_tma && ld % 4 == 0 && aligned)) {
         YKB_TRY_CUDA(launch_fdk_backproject_tma(static_cast<const float*>(filtered), layout, ld,
             coef, count, p->nu, p->nv, grid, p->axial, p->tma_box, vol, accumulate,
-            p->err_flag.as<int>(), p->work_a.as<float>(), p->work_a.bytes / sizeof(float), s,
+            p->err_flag.as<int>(), p->work_filtered.as<float>() + p->filtered_floats, p->part_floats, s,
             nullptr, p->bp_wait));
     } else {
         YKB_TRY_CUDA(launch_fdk_backproject(filtered, YKB_DTYPE_F32, coef, count, p->nu, p->nv,

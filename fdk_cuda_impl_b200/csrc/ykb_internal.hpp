@@ -320,8 +320,11 @@ struct ykb_fdk_plan {
     ykb::DeviceBuffer ramp;      // float[2*nu-1]
     ykb::DeviceBuffer parker;    // float[n_views][nu] short-scan weights, or empty
     ykb::DeviceBuffer toeplitz_hi, toeplitz_lo, toeplitz_lo2;  // bf16 [nu][lda] split parts
-    ykb::DeviceBuffer work_a;    // preweighted rows (float, or the bf16 split parts in turn), then sums of split views
-    ykb::DeviceBuffer work_filtered;  // filtered projections (layout, pitch ld)
+    ykb::DeviceBuffer work_a;    // preweighted rows: float, or the bf16 split parts in turn
+    // filtered projections (layout, pitch ld), filtered_floats of them, then
+    // part_floats for the sums of split views
+    ykb::DeviceBuffer work_filtered;
+    size_t filtered_floats = 0, part_floats = 0;
     ykb::DeviceBuffer err_flag;  // int[8]: device error word, box pre-pass scratch
     // stage timing (ykb_fdk_stage_timing): a start and a stop event around
     // each filter (stage 0) and backprojection (stage 1) launch group, on the
