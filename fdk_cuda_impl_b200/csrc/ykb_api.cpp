@@ -826,7 +826,12 @@ YKB_API ykb_status ykb_joseph_plan_create(const ykb_cone_view* views, int n_view
             e = cudaStreamSynchronize(s);
         p->column_bp = e == cudaSuccess && differs == 0;
         if (!p->column_bp) p->cols.reset();
+        else p->fp_lines = joseph_fp_lines_shape(p->host_views, nv);
     }
+    if (e == cudaSuccess && p->fp_lines.rows > 0 &&
+        (e = p->vt.alloc(sizeof(float) * joseph_line_elems(*volume))) == cudaSuccess &&
+        (e = cudaMemsetAsync(p->vt.ptr, 0, p->vt.bytes, s)) == cudaSuccess)
+        e = cudaStreamSynchronize(s);
     if (e == cudaSuccess)
         e = p->weighted.alloc(sizeof(float) * rays);
     cudaStreamDestroy(s);
@@ -851,7 +856,7 @@ YKB_API size_t ykb_joseph_workspace_bytes(const ykb_joseph_plan* p)
 {
     if (!p) return 0;
     return p->views.bytes + p->view_proj.bytes + p->rays.bytes + p->lens.bytes +
-        p->weighted.bytes + p->cols.bytes + p->slab_x.bytes + p->slab_y.bytes +
+        p->weighted.bytes + p->cols.bytes + p->vt.bytes + p->slab_x.bytes + p->slab_y.bytes +
         p->world_views.bytes +
         p->fdk_coef.bytes +
         p->pseudo_coef.bytes + p->pairs.bytes + p->err_flag.bytes;
@@ -866,6 +871,12 @@ YKB_API ykb_status ykb_joseph_fp(ykb_joseph_plan* p, const float* d_volume, floa
     DeviceGuard guard(p->device);
     const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     const ykb_volume& v = p->volume;
+    if (p->fp_lines.rows > 0) {
+        YKB_TRY_CUDA(launch_joseph_fp_lines(d_volume, v.nx, v.ny, v.nz, p->vt.as<float>(),
+            p->views.as<JosephView>(), p->cols.as<float2>(), p->rays.as<float4>(),
+            p->lens.as<float>(), p->n_views, p->nu, p->nv, p->fp_lines, d_proj, accumulate ? 1 : 0, s));
+        return YKB_OK;
+    }
     YKB_TRY_CUDA(launch_joseph_transpose(d_volume, v.nx, v.ny, v.nz, p->slab_y.as<float>(),
         p->slab_x.as<float>(), s));
     const float* slabs[3] = {p->slab_x.as<float>(), p->slab_y.as<float>(), d_volume};

@@ -263,6 +263,33 @@ cudaError_t launch_joseph_transpose(const float* vol, int nx, int ny, int nz,
 cudaError_t launch_joseph_fp(const float* slabs[3], const JosephView* views,
     const int* view_axis_host, int n_views, int nu, int nv, float* proj,
     int accumulate, cudaStream_t s);
+// Axial-column scans: how far the rays of a view reach over the volume's slices
+// and `margin` voxels around them.  ratio: a voxel's distance from the source
+// over the detector's, along the detector normal.
+struct JosephColumnReach {
+    double near = 0.0, far = 0.0;  // extremes of the ratio
+    double slope = 0.0;            // its change per voxel
+    double pitch = 0.0;            // largest distance along z (voxels) of adjacent rows' rays
+    double tall = 0.0;             // largest height of a detector row over the source (voxels)
+};
+JosephColumnReach joseph_column_reach(const JosephView& j, int nv, double margin);
+// Forward projection of axial-column scans by detector-column lines
+// (joseph_fp_lines.cu): detector rows of a CTA (0: the lines do not fit, the
+// slab kernel projects) and window of its lines
+struct JosephFpLines { int rows = 0, window = 0; };
+JosephFpLines joseph_fp_lines_shape(const std::vector<JosephView>& views, int nv);
+// z pitch (floats) of the volume copy [x][y][z] that the lines are formed from,
+// zero rows around x and y, and its size
+constexpr int kLinePad = 2;
+inline int joseph_line_pitch(int nz) { return (nz + 3) / 4 * 4; }
+inline size_t joseph_line_elems(const ykb_volume& v)
+{
+    return static_cast<size_t>(v.nx + 2 * kLinePad) * (v.ny + 2 * kLinePad) * joseph_line_pitch(v.nz);
+}
+// vt: joseph_line_elems floats, zeroed once; every call rewrites its interior
+cudaError_t launch_joseph_fp_lines(const float* vol, int nx, int ny, int nz, float* vt,
+    const JosephView* views, const float2* cols, const float4* rays, const float* lens, int n_views,
+    int nu, int nv, JosephFpLines shape, float* proj, int accumulate, cudaStream_t s);
 cudaError_t launch_joseph_ray_table(const JosephView* views, int n_views,
     int nu, int nv, float4* rays, float* lens, cudaStream_t s);
 // Iterative-solver vectors (iter_kernels.cu)
@@ -378,6 +405,8 @@ struct ykb_joseph_plan {
     bool column_bp = false;      // every view's detector columns are axial (line backprojector)
     ykb::DeviceBuffer cols;      // float2[n*nu]: (a1, e1) per detector column
     ykb::DeviceBuffer slab_y, slab_x;  // transposed volume copies
+    ykb::JosephFpLines fp_lines;       // forward projection by lines (column_bp scans)
+    ykb::DeviceBuffer vt;              // its volume copy [x][y][z]
     ykb::DeviceBuffer world_views;     // ykb_cone_view[n] (Siddon), uploaded on first use
     // pseudo-matched backprojection, set up on first use
     bool pseudo_ready = false;

@@ -1,0 +1,57 @@
+"""The Joseph line projector (axial-column scans) against the slab projector,
+which takes the same samples with the same weights (YKB_JOSEPH_BP=gather keeps
+it): both round a sample to FP32 and add in FP64, so they differ by the FP32
+rounding of a result.  Sizes at the edges of its groups of 8 detector columns,
+32-row warps, 4-slice batches and 16-byte z quads; rows closer and farther than
+a voxel; views from below (the detector's rows run downwards); a small detector
+that sees part of the volume."""
+import numpy as np
+import pytest
+
+from fdk_cuda_impl_b200.geometry import CircularScan, VolumeGrid
+from tests import cases as K
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # views, nu, nv, pixel u, pixel v, (nx, ny, nz), voxel, flipped
+    (9, 1, 1, 2.0, 2.0, (5, 4, 1), (1.0, 1.0, 1.0), False),
+    (12, 7, 31, 2.0, 2.0, (16, 19, 3), (1.0, 1.0, 1.0), False),
+    (11, 8, 32, 3.0, 3.0, (33, 30, 21), (1.0, 1.2, 0.9), True),
+    (10, 65, 33, 1.1, 1.3, (37, 41, 30), (0.8, 0.9, 1.1), False),
+    (8, 40, 97, 1.6, 0.2, (24, 24, 40), (1.0, 1.0, 1.0), True),     # rows a tenth of a voxel apart
+    (8, 40, 24, 1.6, 9.0, (24, 24, 120), (1.0, 1.0, 1.0), False),   # rows 4.5 voxels apart
+    (8, 24, 130, 1.6, 14.0, (20, 20, 900), (1.0, 1.0, 1.0), False),  # and too far for the lines' window
+    (6, 30, 500, 1.6, 1.6, (40, 36, 420), (1.0, 1.0, 1.0), False),
+]
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_line_projector_matches_slab_projector(oracle, cuda_device, monkeypatch, case):
+    import torch
+    from fdk_cuda_impl_b200.projectors import JosephPlan
+    views, nu, nv, pu, pv, n, vox, flipped = case
+    scan = CircularScan(views, views, 500.0, 1000.0, nu, nv, pu, pv, start_angle_rad=0.05)
+    grid = VolumeGrid(*n, vox, (0.4, -0.7, 0.2))
+    table = scan.views()
+    if flipped:
+        table["detS"][:, :3] += (nv - 1) * table["detV"][:, :3]
+        table["detV"][:, :3] *= -1
+    x = torch.from_numpy(oracle.uniform(grid.shape, 0.0, 1.0, 3)).cuda()
+    lines = JosephPlan(table, nu, nv, grid)
+    monkeypatch.setenv("YKB_JOSEPH_BP", "gather")
+    slabs = JosephPlan(table, nu, nv, grid)
+    a, b = lines.forward(x), slabs.forward(x)
+    assert torch.isfinite(a).all() and float(b.abs().max()) > 0
+    assert K.rel_rmse(a.cpu().numpy(), b.cpu().numpy()) <= 2e-7
+    twice = lines.forward(x, a.clone(), accumulate=True)
+    assert K.rel_rmse(twice.cpu().numpy(), 2 * b.cpu().numpy()) <= 2e-7
+    # a second volume through the same plan: nothing stays of the first
+    y = torch.from_numpy(oracle.uniform(grid.shape, -1.0, 1.0, 4)).cuda()
+    lines.forward(y)
+    assert torch.equal(lines.forward(x), a)
+    if x.numel() < 50000:
+        ref = oracle.joseph_fp(table, nu, nv, K.oracle_volume(oracle, grid), x.cpu().numpy())
+        assert K.rel_rmse(a.cpu().numpy(), ref) <= 1e-5
+    lines.close()
+    slabs.close()
