@@ -161,7 +161,7 @@ __device__ __forceinline__ void slice_span(float a, float e, int n1, int n0, int
 template <int W>
 __global__ void __launch_bounds__(kMaxRows, 2) joseph_fp_lines_kernel(const float* __restrict__ vt,
     const JosephView* __restrict__ views, const float2* __restrict__ cols,
-    const float4* __restrict__ rays, const float* __restrict__ lens, int view0, int nu, int nv,
+    const char* __restrict__ heights, int ray_bytes, const float* __restrict__ lens, int view0, int nu, int nv,
     int nz, int nzp, float* __restrict__ proj, int accumulate)
 {
     extern __shared__ __align__(16) float smem[];
@@ -183,12 +183,13 @@ __global__ void __launch_bounds__(kMaxRows, 2) joseph_fp_lines_kernel(const floa
     // rows and columns past the detector repeat the last one (never stored)
     f2 a2[kCols / 2], e2[kCols / 2];
     {
-        const float4* r = rays + (ray_row + min(iv, nv - 1)) * nu;
+        const char* r = heights + (ray_row + min(iv, nv - 1)) * nu * ray_bytes;
 #pragma unroll
         for (int c = 0; c < kCols; c += 2) {
-            const float4 q = __ldg(r + min(iu0 + c, nu - 1)), p = __ldg(r + min(iu0 + c + 1, nu - 1));
-            a2[c / 2] = f2pack(q.z, p.z);
-            e2[c / 2] = f2pack(q.w, p.w);
+            const float2 q = __ldg(reinterpret_cast<const float2*>(r + min(iu0 + c, nu - 1) * ray_bytes));
+            const float2 p = __ldg(reinterpret_cast<const float2*>(r + min(iu0 + c + 1, nu - 1) * ray_bytes));
+            a2[c / 2] = f2pack(q.x, p.x);
+            e2[c / 2] = f2pack(q.y, p.y);
         }
     }
     // each lane: one column of the table, and a corner ray of the window
@@ -197,9 +198,10 @@ __global__ void __launch_bounds__(kMaxRows, 2) joseph_fp_lines_kernel(const floa
     float ca, ce;
     {
         const int edge = (lane & 8) ? min(row0 + static_cast<int>(blockDim.x) - 1, nv - 1) : row0;
-        const float4 q = __ldg(rays + (ray_row + edge) * nu + min(iu0 + lc, nu - 1));
-        ca = q.z;
-        ce = q.w;
+        const float2 q = __ldg(reinterpret_cast<const float2*>(heights +
+            ((ray_row + edge) * nu + min(iu0 + lc, nu - 1)) * ray_bytes));
+        ca = q.x;
+        ce = q.y;
     }
     const float corner_slice = (lane & 16) ? static_cast<float>(kSlices - 1) : 0.f;
     int slo, shi;
@@ -320,7 +322,7 @@ template <int W> constexpr int lines_smem() { return 2 * 32 * W * 4 + kTables * 
 
 template <int W>
 cudaError_t launch_window(dim3 grid, int threads, const float* vt, const JosephView* views,
-    const float2* cols, const float4* rays, const float* lens, int view0, int nu, int nv, int nz,
+    const float2* cols, JosephHeights heights, const float* lens, int view0, int nu, int nv, int nz,
     int nzp, float* proj, int accumulate, cudaStream_t s)
 {
     constexpr int smem = lines_smem<W>();
@@ -330,7 +332,7 @@ cudaError_t launch_window(dim3 grid, int threads, const float* vt, const JosephV
     // the CTAs of an SM share 200 KB of it
     e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 88);
     if (e != cudaSuccess) return e;
-    k<<<grid, threads, smem, s>>>(vt, views, cols, rays, lens, view0, nu, nv, nz, nzp, proj, accumulate);
+    k<<<grid, threads, smem, s>>>(vt, views, cols, heights.first, heights.bytes, lens, view0, nu, nv, nz, nzp, proj, accumulate);
     return cudaGetLastError();
 }
 
@@ -358,6 +360,20 @@ JosephColumnReach joseph_column_reach(const JosephView& j, int nv, double margin
     r.tall = std::max(std::fabs(j.detS[2] - j.src[2]),
         std::fabs(j.detS[2] + (nv - 1) * j.detV[2] - j.src[2]));
     return r;
+}
+
+// A ray of a line reaches at most a voxel past the volume on the minor axis and
+// the slice of a pair past the last one; 4 voxels cover both.  0.999 and 0.001:
+// two roundings of a coordinate below 2^13 voxels.
+bool joseph_bp_runs(const std::vector<JosephView>& views, int nv)
+{
+    for (const JosephView& j : views) {
+        const JosephColumnReach r = joseph_column_reach(j, nv, 4.0);
+        if (!(r.near > 0.0) || !(r.pitch <= 0.999) || !(std::fabs(j.detV[2]) * r.near >= 1e-3) ||
+            j.n2 > 8192)
+            return false;
+    }
+    return true;
 }
 
 // Rows of a CTA and window of its lines, from the largest spread of the rays of
@@ -397,7 +413,7 @@ JosephFpLines joseph_fp_lines_shape(const std::vector<JosephView>& views, int nv
 }
 
 cudaError_t launch_joseph_fp_lines(const float* vol, int nx, int ny, int nz, float* vt,
-    const JosephView* views, const float2* cols, const float4* rays, const float* lens, int n_views,
+    const JosephView* views, const float2* cols, JosephHeights heights, const float* lens, int n_views,
     int nu, int nv, JosephFpLines shape, float* proj, int accumulate, cudaStream_t s)
 {
     const int nzp = joseph_line_pitch(nz);
@@ -421,7 +437,7 @@ cudaError_t launch_joseph_fp_lines(const float* vol, int nx, int ny, int nz, flo
         case 304: launch = launch_window<304>; break;
         default: launch = launch_window<400>; break;
         }
-        e = launch(grid, shape.rows, vt, views, cols, rays, lens, done, nu, nv, nz, nzp, proj,
+        e = launch(grid, shape.rows, vt, views, cols, heights, lens, done, nu, nv, nz, nzp, proj,
             accumulate, s);
     }
     return e;

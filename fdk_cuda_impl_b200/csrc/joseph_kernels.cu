@@ -185,6 +185,20 @@ __device__ __forceinline__ f2 f2sub(f2 a, f2 b)
     return d;
 }
 
+// rounded towards minus infinity
+__device__ __forceinline__ f2 f2add_rm(f2 a, f2 b)
+{
+    f2 d;
+    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f2 f2mul(f2 a, f2 b)
+{
+    f2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
 // 1.5 * 2^23: for |x| < 2^22, x + kMagic holds round(x) in its low mantissa
 // bits; (f - 1/2) + kMagic thus holds floor(f), except at integer f where
 // it may hold f - 1 -- with fraction 1, the same bilinear weights.
@@ -378,6 +392,23 @@ __device__ __forceinline__ void footprint_box(const ViewProj& m, const JosephVie
     footprint_box_range(m, j, c0, j1, j1, j2lo, j2hi, nu, nv, u0, u1, v0, v1);
 }
 
+// Detector columns of [j1 - 1, j1 + 1] on slice c0 of an axial-column scan, whose
+// u does not depend on z (m[2] = m[10] = 0)
+__device__ __forceinline__ void column_span(const ViewProj& m, const JosephView& j, float c0, int j1,
+    int nu, int& u0, int& u1)
+{
+    const float q = static_cast<float>(j1) - 0.5f * (j.n1 - 1);
+    const bool ax0 = j.axis == 0;
+    // numerator and denominator: along the minor axis, and at (c0, 0)
+    const float n1 = ax0 ? m.m[1] : m.m[0], n0 = fmaf(ax0 ? m.m[0] : m.m[1], c0, m.m[3]);
+    const float d1 = ax0 ? m.m[9] : m.m[8], d0 = fmaf(ax0 ? m.m[8] : m.m[9], c0, m.m[11]);
+    const float ua = fmaf(n1, q - 1.f, n0) * __frcp_rn(fmaf(d1, q - 1.f, d0));
+    const float ub = fmaf(n1, q + 1.f, n0) * __frcp_rn(fmaf(d1, q + 1.f, d0));
+    constexpr float margin = 0.05f;
+    u0 = max(0, static_cast<int>(ceilf(fminf(ua, ub) - margin)));
+    u1 = min(nu - 1, static_cast<int>(floorf(fmaxf(ua, ub) + margin)));
+}
+
 // One thread gathers ZV voxels stacked along z.  When z is a minor axis of
 // the view (main axis x or y, every view of a circular orbit) the stack lies
 // in one slice with a common minor-1 index: each candidate ray of the stack's
@@ -525,6 +556,25 @@ constexpr int kLineMax = 32;      // lines of a slice per pass
 template <int ZC>
 __host__ __device__ constexpr int line_slice_words() { return (ZC + 2) * kLineMax + 21; }
 
+// CTAs over z blocks, then over splits of the views: with more than one split
+// each writes its FP64 sums to parts[split], which sum_line_parts_kernel adds
+struct LineSplits {
+    int z_blocks, splits;
+    double* parts;
+};
+
+// out[i] (+)= the sum of the splits' parts, in order
+__global__ void __launch_bounds__(256) sum_line_parts_kernel(const double* __restrict__ parts, int splits,
+    long n, float* __restrict__ out, int accumulate)
+{
+    for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < n;
+         i += static_cast<long>(gridDim.x) * blockDim.x) {
+        double a = accumulate ? out[i] : 0.0;
+        for (int s = 0; s < splits; ++s) a += __ldcs(parts + s * n + i);
+        out[i] = static_cast<float>(a);
+    }
+}
+
 template <int ZC>
 constexpr size_t line_smem_bytes()
 {
@@ -536,7 +586,7 @@ template <int ZC>
 __global__ void __launch_bounds__(kLineThreads, 3) joseph_bp_lines_kernel(
     const float4* __restrict__ rays, const float* __restrict__ wv, const float2* __restrict__ cols,
     const ViewProj* __restrict__ vp, const JosephView* __restrict__ views, int n_views, int nu,
-    int nv, int nx, int ny, int nz, float* __restrict__ vol, int accumulate)
+    int nv, int nx, int ny, int nz, LineSplits sp, float* __restrict__ vol, int accumulate)
 {
     constexpr int B = kLineBlock, SL = ZC + 2, LM = kLineMax, PS = line_slice_words<ZC>();
     extern __shared__ __align__(16) unsigned char line_smem[];
@@ -550,7 +600,10 @@ __global__ void __launch_bounds__(kLineThreads, 3) joseph_bp_lines_kernel(
         (reinterpret_cast<uintptr_t>(lines + B * PS) + 15) & ~static_cast<uintptr_t>(15));
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tx = tid % B, ty = tid / B;
-    const int X0 = blockIdx.x * B, Y0 = blockIdx.y * B, z0 = blockIdx.z * ZC;
+    const int split = blockIdx.z / sp.z_blocks;
+    const int X0 = blockIdx.x * B, Y0 = blockIdx.y * B, z0 = (blockIdx.z - split * sp.z_blocks) * ZC;
+    const int k0 = static_cast<int>(static_cast<long>(n_views) * split / sp.splits);
+    const int k1 = static_cast<int>(static_cast<long>(n_views) * (split + 1) / sp.splits);
     const int x = X0 + tx, y = Y0 + ty;
     const bool mine = x < nx && y < ny;
 #pragma unroll
@@ -561,7 +614,7 @@ __global__ void __launch_bounds__(kLineThreads, 3) joseph_bp_lines_kernel(
     float acc[ZC];  // FP32 over sixteen views, then into the FP64 sums
 #pragma unroll
     for (int q = 0; q < ZC; ++q) acc[q] = 0.f;
-    for (int k = 0; k < n_views; ++k) {
+    for (int k = k0; k < k1; ++k) {
         const JosephView& j = views[k];
         const bool ax0 = j.axis == 0;
         const int S0 = ax0 ? X0 : Y0, J0 = ax0 ? Y0 : X0;  // first slice, first minor-1 index
@@ -600,8 +653,8 @@ __global__ void __launch_bounds__(kLineThreads, 3) joseph_bp_lines_kernel(
         // this thread's voxel column: its slice, minor-1 index, candidates
         const int pl = ax0 ? tx : ty, j1 = ax0 ? y : x;
         const float c0 = static_cast<float>(S0 + pl) - half;
-        int cu0 = 0, cu1 = -1, cv0, cv1;
-        if (mine) footprint_box(vp[k], j, c0, j1, z0, z0 + ZC - 1, nu, nv, cu0, cu1, cv0, cv1);
+        int cu0 = 0, cu1 = -1;
+        if (mine) column_span(vp[k], j, c0, j1, nu, cu0, cu1);
         const float j1f = static_cast<float>(j1);
         const float2* ck = cols + static_cast<long>(k) * nu;
         for (int pass = 0; pass < passes; ++pass) {
@@ -683,7 +736,7 @@ __global__ void __launch_bounds__(kLineThreads, 3) joseph_bp_lines_kernel(
             }
             __syncthreads();
         }
-        if ((k & 15) == 15 || k + 1 == n_views) {
+        if (((k - k0) & 15) == 15 || k + 1 == k1) {
 #pragma unroll
             for (int q = 0; q < ZC; ++q) {
                 total[q * kLineThreads + tid] += static_cast<double>(acc[q]);
@@ -696,13 +749,334 @@ __global__ void __launch_bounds__(kLineThreads, 3) joseph_bp_lines_kernel(
 #pragma unroll
     for (int q = 0; q < ZC; ++q) {
         if (z0 + q >= nz) break;
-        float* dst = vol + (z0 + q) * plane + static_cast<long>(y) * nx + x;
+        const long at = (z0 + q) * plane + static_cast<long>(y) * nx + x;
         const double a = total[q * kLineThreads + tid];
+        if (sp.splits > 1) {
+            sp.parts[split * plane * nz + at] = a;
+            continue;
+        }
+        float* dst = vol + at;
         *dst = accumulate ? static_cast<float>(*dst + a) : static_cast<float>(a);
     }
 }
 
+// ---------------------------------------------------------------------------
+// The line backprojector for scans whose adjacent rows' rays are less than a
+// voxel apart along z everywhere (joseph_bp_runs: every scan whose detector
+// resolves the voxels).  The same lines, block and column sums as
+// joseph_bp_lines_kernel; here
+//   * a column's rays visit its line's voxels in runs, so an entry is two sums
+//     in registers and one store per ray instead of two reads and two writes of
+//     shared memory (a voxel's entry is stored with every ray of its run, the
+//     last one leaving it complete);
+//   * the lines of all slice pairs are dealt to the threads in turn (about 26
+//     detector columns reach a pair's 16 voxels, so a warp a pair leaves a fifth
+//     of its lanes idle);
+//   * the last warp, which the lines rarely reach, prepares the next view's
+//     boxes, and every thread has its next line's first rays in flight while it
+//     sums its column: two barriers a view.
+// ---------------------------------------------------------------------------
+constexpr int kRunGroup = 4;  // rays of a line loaded together
+
+// words from one slice's lines to the next: 13 mod 32.  A pair's lines fill about
+// 26 lanes and banks, and the next pair's begin 26 banks on; a warp's column sums
+// read two slices (16 lanes each, over some 20 banks) or sixteen (distinct odd
+// multiples).  An order of its own for each main axis, 1.7 wavefronts a request of
+// the column sums instead of 3, measured 6 % slower (22.8 ms): its stores and
+// addresses cost more
+template <int ZC>
+__host__ __device__ constexpr int run_slice_words() { return (ZC + 2) * kLineMax + 13; }
+
+// a view's line boxes: u0, u1, v0, v1 of each slice pair, the number of lines
+// of the pairs before each (first pass), and the passes
+struct RunView {
+    int4 box[kLineBlock / 2];
+    int before[kLineBlock / 2];
+    int passes;
+    int pad[3];
+};
+
+template <int ZC>
+constexpr size_t run_smem_bytes()
+{
+    return sizeof(double) * ZC * kLineThreads +
+        sizeof(float) * kLineBlock * (run_slice_words<ZC>() + kLineMax) + 16 + 2 * sizeof(RunView);
+}
+
+// one warp: the boxes of a view for the block at (X0, Y0, z0)
+template <int ZC>
+__device__ __forceinline__ void prepare_run_view(RunView& out, const ViewProj& m, const JosephView& j,
+    int X0, int Y0, int z0, int nu, int nv)
+{
+    constexpr int B = kLineBlock;
+    const int lane = threadIdx.x & 31;
+    const bool ax0 = j.axis == 0;
+    const int S0 = ax0 ? X0 : Y0, J0 = ax0 ? Y0 : X0;
+    const int nS = min(B, j.n0 - S0), nJ = min(B, j.n1 - J0);
+    int u0 = 0x7fffffff, u1 = -0x7fffffff, v0 = 0x7fffffff, v1 = -0x7fffffff;
+    if (lane < nS) {
+        int a, b, c, d;
+        footprint_box_range(m, j, static_cast<float>(S0 + lane) - 0.5f * (j.n0 - 1), J0, J0 + nJ - 1, z0,
+            z0 + ZC - 1, nu, nv, a, b, c, d);
+        if (a <= b && c <= d) { u0 = a; u1 = b; v0 = c; v1 = d; }
+    }
+    // the two slices of a pair share the union of their boxes: a ray outside a
+    // slice's own box adds nothing to the lines its voxel columns read
+    u0 = min(u0, __shfl_xor_sync(0xffffffffu, u0, 1));
+    u1 = max(u1, __shfl_xor_sync(0xffffffffu, u1, 1));
+    v0 = min(v0, __shfl_xor_sync(0xffffffffu, v0, 1));
+    v1 = max(v1, __shfl_xor_sync(0xffffffffu, v1, 1));
+    const int n = u0 <= u1 ? u1 - u0 + 1 : 0;
+    int sum = (lane & 1) || lane >= B ? 0 : min(n, kLineMax);
+    const int own = sum;
+#pragma unroll
+    for (int o = 2; o < B; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += t;
+    }
+    const int most = __reduce_max_sync(0xffffffffu, lane < B ? n : 0);
+    if (lane < B && !(lane & 1)) {
+        out.box[lane / 2] = n > 0 ? make_int4(u0, u1, v0, v1) : make_int4(0, -1, 0, -1);
+        out.before[lane / 2] = sum - own;
+    }
+    if (lane == 0) out.passes = (most + kLineMax - 1) / kLineMax;
+}
+
+// a thread's line: its first ray, step to the next, number of rays, pair and
+// column (count 0: none)
+struct RunLine {
+    int first, step, count, pair, column;
+};
+
+__device__ __forceinline__ RunLine run_line(const RunView& rv, int pass, bool up, int nu)
+{
+    constexpr int P = kLineBlock / 2;
+    RunLine l;
+    int pair = 0, c = threadIdx.x;
+    if (pass == 0) {
+        const int4 lo = *reinterpret_cast<const int4*>(&rv.before[0]);
+        const int4 hi = *reinterpret_cast<const int4*>(&rv.before[4]);
+        static_assert(P == 8, "two loads");
+        const int t = c;
+        pair = (t >= lo.y) + (t >= lo.z) + (t >= lo.w) + (t >= hi.x) + (t >= hi.y) + (t >= hi.z) + (t >= hi.w);
+        c -= rv.before[pair];
+    } else {
+        for (; pair < P - 1; ++pair) {
+            const int here = min(max(rv.box[pair].y - rv.box[pair].x + 1 - pass * kLineMax, 0), kLineMax);
+            if (c < here) break;
+            c -= here;
+        }
+    }
+    const int4 b = rv.box[pair];
+    const int iu = b.x + pass * kLineMax + c;
+    l.pair = pair;
+    l.column = c;
+    l.count = c < kLineMax && iu <= b.y ? b.w - b.z + 1 : 0;
+    l.first = (up ? b.z : b.w) * nu + iu;
+    l.step = up ? nu : -nu;
+    return l;
+}
+
+struct RunRays {
+    float2 a[kRunGroup];
+    float v[kRunGroup];
+};
+
+// rays i .. i + 3 of a line; past its last ray, that one with value zero
+__device__ __forceinline__ void load_rays(RunRays& r, const char* rays, int ray_bytes, const float* wv,
+    const RunLine& l, int i)
+{
+#pragma unroll
+    for (int q = 0; q < kRunGroup; ++q) {
+        const bool in = i + q < l.count;
+        const int at = l.first + (in ? i + q : l.count - 1) * l.step;
+        r.a[q] = __ldg(reinterpret_cast<const float2*>(rays + static_cast<long>(at) * ray_bytes));
+        r.v[q] = in ? __ldg(wv + at) : 0.f;
+    }
+}
+
+template <int ZC>
+__global__ void __launch_bounds__(kLineThreads, 3) joseph_bp_runs_kernel(
+    const char* __restrict__ rays, int ray_bytes, const float* __restrict__ wv, const float2* __restrict__ cols,
+    const ViewProj* __restrict__ vp, const JosephView* __restrict__ views, int n_views, int nu,
+    int nv, int nx, int ny, int nz, LineSplits sp, float* __restrict__ vol, int accumulate)
+{
+    constexpr int B = kLineBlock, LM = kLineMax, PS = run_slice_words<ZC>();
+    extern __shared__ __align__(16) unsigned char line_smem[];
+    double* total = reinterpret_cast<double*>(line_smem);                 // [q][thread]
+    float* lines = reinterpret_cast<float*>(total + ZC * kLineThreads);  // [slice][slot][line]
+    float* places = lines + B * PS;                                       // [slice][line]: f1
+    RunView* rviews = reinterpret_cast<RunView*>(
+        (reinterpret_cast<uintptr_t>(places + B * LM) + 15) & ~static_cast<uintptr_t>(15));
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tx = tid % B, ty = tid / B;
+    const int split = blockIdx.z / sp.z_blocks;
+    const int X0 = blockIdx.x * B, Y0 = blockIdx.y * B, z0 = (blockIdx.z - split * sp.z_blocks) * ZC;
+    const int k0 = static_cast<int>(static_cast<long>(n_views) * split / sp.splits);
+    const int k1 = static_cast<int>(static_cast<long>(n_views) * (split + 1) / sp.splits);
+    const int x = X0 + tx, y = Y0 + ty;
+    const bool mine = x < nx && y < ny;
+    const int view_rays = nu * nv;
+    constexpr int kLast = kLineThreads / 32 - 1;
+#pragma unroll
+    for (int q = 0; q < ZC; ++q) total[q * kLineThreads + tid] = 0.0;
+    // slot of floor(f2) + 1 from the floor word of f2 (wrapping)
+    const uint32_t slot0 = kMagicBits + static_cast<uint32_t>(z0 - 1);
+    const f2 M = f2pack(kMagic, kMagic);
+    float acc[ZC];  // FP32 over sixteen views, then into the FP64 sums
+#pragma unroll
+    for (int q = 0; q < ZC; ++q) acc[q] = 0.f;
+    if (warp == kLast) prepare_run_view<ZC>(rviews[k0 & 1], vp[k0], views[k0], X0, Y0, z0, nu, nv);
+    __syncthreads();
+    RunLine line = run_line(rviews[k0 & 1], 0, views[k0].detV[2] > 0.0, nu);
+    RunRays next;
+    if (line.count > 0)
+        load_rays(next, rays + static_cast<long>(k0) * view_rays * ray_bytes, ray_bytes,
+            wv + static_cast<long>(k0) * view_rays, line, 0);
+    for (int k = k0; k < k1; ++k) {
+        const JosephView& j = views[k];
+        const RunView& rv = rviews[k & 1];
+        const bool ax0 = j.axis == 0;
+        const int S0 = ax0 ? X0 : Y0;
+        const float half = 0.5f * (j.n0 - 1);
+        const char* rk = rays + static_cast<long>(k) * view_rays * ray_bytes;
+        const float* wk = wv + static_cast<long>(k) * view_rays;
+        const int passes = rv.passes;
+        const bool up = j.detV[2] > 0.0;  // f2 grows with the row
+        // this thread's voxel column: its slice, minor-1 index, candidates
+        const int pl = ax0 ? tx : ty, j1 = ax0 ? y : x;
+        const float c0 = static_cast<float>(S0 + pl) - half;
+        const float j1f = static_cast<float>(j1);
+        int cu0 = 0, cu1 = -1;
+        if (mine) column_span(vp[k], j, c0, j1, nu, cu0, cu1);
+        for (int pass = 0; pass < max(passes, 1); ++pass) {
+            if (pass > 0) {
+                line = run_line(rv, pass, up, nu);
+                if (line.count > 0) load_rays(next, rk, ray_bytes, wk, line, 0);
+            }
+            // ---- this thread's line, on both slices of its pair
+            if (line.count > 0) {
+                float* const La = lines + 2 * line.pair * PS + line.column;
+                float* const Lb = La + PS;
+                const float csa = static_cast<float>(S0 + 2 * line.pair) - half, csb = csa + 1.f;
+                {
+                    // the line's minor-1 positions, for the column sums
+                    const float2 ce = __ldg(cols + static_cast<long>(k) * nu + rv.box[line.pair].x +
+                        pass * LM + line.column);
+                    float* at = places + 2 * line.pair * LM + line.column;
+                    at[0] = fmaf(ce.x, csa, ce.y);
+                    at[LM] = fmaf(ce.x, csb, ce.y);
+                }
+                float cur[2], lo[2] = {0.f, 0.f}, hi[2] = {0.f, 0.f};
+                cur[0] = __fadd_rd(fmaf(next.a[0].x, csa, next.a[0].y), kMagic);
+                cur[1] = __fadd_rd(fmaf(next.a[0].x, csb, next.a[0].y), kMagic);
+                const int start[2] = {static_cast<int>(__float_as_uint(cur[0]) - slot0),
+                                      static_cast<int>(__float_as_uint(cur[1]) - slot0)};
+                for (int i = 0; i < line.count; i += kRunGroup) {
+                    const RunRays r = next;
+                    if (i + kRunGroup < line.count) load_rays(next, rk, ray_bytes, wk, line, i + kRunGroup);
+#pragma unroll
+                    for (int q = 0; q < kRunGroup; ++q) {
+                        const f2 f = f2pack(fmaf(r.a[q].x, csa, r.a[q].y), fmaf(r.a[q].x, csb, r.a[q].y));
+                        const f2 t = f2add_rm(f, M);
+                        const f2 vv = f2pack(r.v[q], r.v[q]), u = f2mul(vv, f2sub(f, f2sub(t, M)));
+                        float tt[2], uu[2], xx[2];
+                        f2unpack(t, tt[0], tt[1]);
+                        f2unpack(u, uu[0], uu[1]);
+                        f2unpack(f2sub(vv, u), xx[0], xx[1]);
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const bool begins = tt[e] != cur[e];  // the next voxel
+                            lo[e] = (begins ? hi[e] : lo[e]) + xx[e];
+                            hi[e] = (begins ? 0.f : hi[e]) + uu[e];
+                            cur[e] = tt[e];
+                            // slot ZC + 1 takes what falls outside
+                            const uint32_t slot = min(__float_as_uint(tt[e]) - slot0,
+                                static_cast<uint32_t>(ZC + 1));
+                            (e ? Lb : La)[slot * LM] = lo[e];
+                        }
+                    }
+                }
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    // the entry after the last ray's; entries no ray reaches are zero
+                    float* const L = e ? Lb : La;
+                    const int last = static_cast<int>(__float_as_uint(cur[e]) - slot0);
+                    if (last >= 0 && last < ZC) L[(last + 1) * LM] = hi[e];
+                    for (int q = min(start[e] - 1, ZC); q >= 1; --q) L[q * LM] = 0.f;
+                    for (int q = max(last + 2, 1); q <= ZC; ++q) L[q * LM] = 0.f;
+                }
+            }
+            // the next view's boxes: its slot was last read before the previous
+            // view's second barrier
+            if (pass == 0 && warp == kLast && k + 1 < k1)
+                prepare_run_view<ZC>(rviews[(k + 1) & 1], vp[k + 1], views[k + 1], X0, Y0, z0, nu, nv);
+            __syncthreads();
+            // the next view's first rays, in flight during the sums
+            if (pass + 1 >= passes && k + 1 < k1) {
+                line = run_line(rviews[(k + 1) & 1], 0, views[k + 1].detV[2] > 0.0, nu);
+                if (line.count > 0) 
+                    load_rays(next, rk + static_cast<long>(view_rays) * ray_bytes, ray_bytes,
+                        wk + view_rays, line, 0);
+            }
+            // ---- this column: its candidates among this pass's lines
+            if (mine) {
+                const int4 b = rv.box[pl >> 1];
+                const int base = b.x + pass * LM;
+                const int lo = max(cu0, base), hi = min(min(cu1, b.y), base + LM - 1);
+                const float* Lp = lines + pl * PS - base;
+                const float* fp = places + pl * LM - base;
+                for (int iu = lo; iu <= hi; ++iu) {
+                    // the forward projector's minor-1 weights (see hat_weight)
+                    const float h1 = __saturatef(1.f - fabsf(fp[iu] - j1f));
+                    if (h1 == 0.f) continue;
+#pragma unroll
+                    for (int q = 0; q < ZC; ++q) acc[q] = fmaf(h1, Lp[(q + 1) * LM + iu], acc[q]);
+                }
+            }
+            __syncthreads();
+        }
+        if (((k - k0) & 15) == 15 || k + 1 == k1) {
+#pragma unroll
+            for (int q = 0; q < ZC; ++q) {
+                total[q * kLineThreads + tid] += static_cast<double>(acc[q]);
+                acc[q] = 0.f;
+            }
+        }
+    }
+    if (!mine) return;
+    const long plane = static_cast<long>(nx) * ny;
+#pragma unroll
+    for (int q = 0; q < ZC; ++q) {
+        if (z0 + q >= nz) break;
+        const long at = (z0 + q) * plane + static_cast<long>(y) * nx + x;
+        const double a = total[q * kLineThreads + tid];
+        if (sp.splits > 1) {
+            sp.parts[split * plane * nz + at] = a;
+            continue;
+        }
+        float* dst = vol + at;
+        *dst = accumulate ? static_cast<float>(*dst + a) : static_cast<float>(a);
+    }
+}
+
+// (a2, e2) of every ray from its record
+__global__ void joseph_ray_heights_kernel(const float4* __restrict__ rays, long n, float2* __restrict__ out)
+{
+    for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < n;
+         i += static_cast<long>(gridDim.x) * blockDim.x) {
+        const float4 r = rays[i];
+        out[i] = make_float2(r.z, r.w);
+    }
+}
+
 } // namespace
+
+cudaError_t launch_joseph_ray_heights(const float4* rays, long n, float2* out, cudaStream_t s)
+{
+    joseph_ray_heights_kernel<<<148 * 8, 256, 0, s>>>(rays, n, out);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_joseph_column_table(const float4* rays, int n_views, int nu, int nv,
     float2* cols, int* flag, cudaStream_t s)
@@ -715,24 +1089,60 @@ cudaError_t launch_joseph_column_table(const float4* rays, int n_views, int nu, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_joseph_bp_lines(const float* proj, const float4* rays, const float* lens,
-    const float2* cols, const float* view_proj, const JosephView* views, int n_views, int nu,
-    int nv, const ykb_volume& vol, float* weighted, float* out, int accumulate, cudaStream_t s)
+// Splits of the views that finish the line backprojector soonest: three CTAs of
+// 16 x 16 x 16 voxels an SM, 6 us a CTA and view, two views' time to start and
+// end, and the splits' sums (4 us, a write and a read at 4 TB/s, at most 64 MB).
+// 64 x 64 x 48 x 60 views, 48 blocks: 52 us in nine splits, 259 in one
+int joseph_bp_splits(const ykb_volume& v, int n_views)
+{
+    const long blocks = static_cast<long>((v.nx + kLineBlock - 1) / kLineBlock) *
+        ((v.ny + kLineBlock - 1) / kLineBlock) * ((v.nz + 15) / 16);
+    const double bytes = 8.0 * v.nx * v.ny * v.nz;
+    int best = 1;
+    double best_cost = 0.0;
+    for (int s = 1; s <= 32 && (s == 1 || (4 * s <= n_views && s * bytes <= 64e6)); ++s) {
+        double cost = static_cast<double>((blocks * s + 443) / 444) * ((n_views + s - 1) / s + 2.0) * 6e-6;
+        if (s > 1) cost += 4e-6 + 2.0 * s * bytes / 4e12;
+        if (s == 1 || cost < best_cost) {
+            best = s;
+            best_cost = cost;
+        }
+    }
+    return best;
+}
+
+cudaError_t launch_joseph_bp_lines(const float* proj, const float4* rays, JosephHeights heights,
+    const float* lens, const float2* cols, const float* view_proj, const JosephView* views, int n_views,
+    int nu, int nv, const ykb_volume& vol, bool runs, float* weighted, int splits, double* parts, float* out,
+    int accumulate, cudaStream_t s)
 {
     const long n = static_cast<long>(n_views) * nu * nv;
     joseph_weight_rays_kernel<<<148 * 8, 256, 0, s>>>(proj, lens, n, weighted);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     constexpr int ZC = 16;
-    auto k = joseph_bp_lines_kernel<ZC>;
-    constexpr size_t smem = line_smem_bytes<ZC>();
-    if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-             static_cast<int>(smem))) != cudaSuccess)
+    const size_t smem = runs ? run_smem_bytes<ZC>() : line_smem_bytes<ZC>();
+    if ((e = cudaFuncSetAttribute(runs ? reinterpret_cast<const void*>(joseph_bp_runs_kernel<ZC>)
+                                       : reinterpret_cast<const void*>(joseph_bp_lines_kernel<ZC>),
+             cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem))) != cudaSuccess)
         return e;
+    const int z_blocks = (vol.nz + ZC - 1) / ZC;
     const dim3 grid((vol.nx + kLineBlock - 1) / kLineBlock, (vol.ny + kLineBlock - 1) / kLineBlock,
-        (vol.nz + ZC - 1) / ZC);
-    k<<<grid, kLineThreads, smem, s>>>(rays, weighted, cols, reinterpret_cast<const ViewProj*>(view_proj),
-        views, n_views, nu, nv, vol.nx, vol.ny, vol.nz, out, accumulate);
+        z_blocks * splits);
+    const LineSplits sp{z_blocks, splits, parts};
+    const ViewProj* vp = reinterpret_cast<const ViewProj*>(view_proj);
+    if (runs)
+        joseph_bp_runs_kernel<ZC><<<grid, kLineThreads, smem, s>>>(heights.first, heights.bytes, weighted,
+            cols, vp, views, n_views, nu, nv, vol.nx, vol.ny, vol.nz, sp, out, accumulate);
+    else
+        joseph_bp_lines_kernel<ZC><<<grid, kLineThreads, smem, s>>>(rays, weighted, cols, vp, views, n_views,
+            nu, nv, vol.nx, vol.ny, vol.nz, sp, out, accumulate);
+    if (splits > 1) {
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        const long voxels = static_cast<long>(vol.nx) * vol.ny * vol.nz;
+        sum_line_parts_kernel<<<static_cast<unsigned>(min((voxels + 255) / 256, 148 * 8L)), 256, 0, s>>>(
+            parts, splits, voxels, out, accumulate);
+    }
     return cudaGetLastError();
 }
 

@@ -783,9 +783,7 @@ YKB_API ykb_status ykb_joseph_plan_create(const ykb_cone_view* views, int n_view
     if ((e = p->views.alloc(sizeof(JosephView) * n_views)) != cudaSuccess ||
         (e = p->view_proj.alloc(sizeof(float) * vp.size())) != cudaSuccess ||
         (e = p->rays.alloc(sizeof(float4) * rays)) != cudaSuccess ||
-        (e = p->lens.alloc(sizeof(float) * rays)) != cudaSuccess ||
-        (need_y && (e = p->slab_y.alloc(sizeof(float) * joseph_slab_elems(*volume, 1))) != cudaSuccess) ||
-        (need_x && (e = p->slab_x.alloc(sizeof(float) * joseph_slab_elems(*volume, 0))) != cudaSuccess)) {
+        (e = p->lens.alloc(sizeof(float) * rays)) != cudaSuccess) {
         delete p;
         return cuda_status(e, "cudaMalloc (Joseph plan)");
     }
@@ -802,12 +800,8 @@ YKB_API ykb_status ykb_joseph_plan_create(const ykb_cone_view* views, int n_view
         delete p;
         return cuda_status(e, "cudaStreamCreate");
     }
-    // the slabs' zero borders, written once (the transposes fill the interior)
-    if (p->slab_y.ptr) e = cudaMemsetAsync(p->slab_y.ptr, 0, p->slab_y.bytes, s);
-    if (e == cudaSuccess && p->slab_x.ptr) e = cudaMemsetAsync(p->slab_x.ptr, 0, p->slab_x.bytes, s);
-    if (e == cudaSuccess)
-        e = launch_joseph_ray_table(p->views.as<JosephView>(), n_views, nu, nv,
-            p->rays.as<float4>(), p->lens.as<float>(), s);
+    e = launch_joseph_ray_table(p->views.as<JosephView>(), n_views, nu, nv,
+        p->rays.as<float4>(), p->lens.as<float>(), s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     // the line backprojector when every view's main axis is x or y and its
     // detector columns are axial (YKB_JOSEPH_BP=gather keeps the gather)
@@ -826,14 +820,41 @@ YKB_API ykb_status ykb_joseph_plan_create(const ykb_cone_view* views, int n_view
             e = cudaStreamSynchronize(s);
         p->column_bp = e == cudaSuccess && differs == 0;
         if (!p->column_bp) p->cols.reset();
-        else p->fp_lines = joseph_fp_lines_shape(p->host_views, nv);
+        if (p->column_bp) {
+            p->fp_lines = joseph_fp_lines_shape(p->host_views, nv);
+            p->bp_runs = joseph_bp_runs(p->host_views, nv);
+            // without room for the table the ray records serve
+            if (p->heights.alloc(sizeof(float2) * rays) == cudaSuccess)
+                e = launch_joseph_ray_heights(p->rays.as<float4>(), static_cast<long>(rays),
+                    p->heights.as<float2>(), s);
+            else
+                cudaGetLastError();
+        }
     }
-    if (e == cudaSuccess && p->fp_lines.rows > 0 &&
-        (e = p->vt.alloc(sizeof(float) * joseph_line_elems(*volume))) == cudaSuccess &&
-        (e = cudaMemsetAsync(p->vt.ptr, 0, p->vt.bytes, s)) == cudaSuccess)
-        e = cudaStreamSynchronize(s);
-    if (e == cudaSuccess)
-        e = p->weighted.alloc(sizeof(float) * rays);
+    // the forward projector's volume copies, their zero borders written once (the
+    // transposes fill the interior)
+    if (p->fp_lines.rows > 0) need_x = need_y = false;
+    const auto zeroed = [&](DeviceBuffer& b, size_t floats) {
+        if (e == cudaSuccess && (e = b.alloc(sizeof(float) * floats)) == cudaSuccess)
+            e = cudaMemsetAsync(b.ptr, 0, b.bytes, s);
+    };
+    if (need_y) zeroed(p->slab_y, joseph_slab_elems(*volume, 1));
+    if (need_x) zeroed(p->slab_x, joseph_slab_elems(*volume, 0));
+    if (p->fp_lines.rows > 0) zeroed(p->vt, joseph_line_elems(*volume));
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) {
+        // behind the weighted rays, the sums of split views; without room for
+        // them the views are not split
+        const size_t weighted = (sizeof(float) * rays + 255) / 256 * 256;
+        if (p->column_bp) p->bp_splits = joseph_bp_splits(*volume, n_views);
+        if (p->bp_splits > 1 && p->weighted.alloc(weighted +
+                sizeof(double) * p->bp_splits * volume_elems(*volume)) != cudaSuccess) {
+            cudaGetLastError();
+            p->bp_splits = 1;
+        }
+        if (p->bp_splits > 1) p->bp_parts = reinterpret_cast<double*>(p->weighted.as<char>() + weighted);
+        else e = p->weighted.alloc(weighted);
+    }
     cudaStreamDestroy(s);
     if (e != cudaSuccess) {
         delete p;
@@ -856,7 +877,7 @@ YKB_API size_t ykb_joseph_workspace_bytes(const ykb_joseph_plan* p)
 {
     if (!p) return 0;
     return p->views.bytes + p->view_proj.bytes + p->rays.bytes + p->lens.bytes +
-        p->weighted.bytes + p->cols.bytes + p->vt.bytes + p->slab_x.bytes + p->slab_y.bytes +
+        p->weighted.bytes + p->cols.bytes + p->heights.bytes + p->vt.bytes + p->slab_x.bytes + p->slab_y.bytes +
         p->world_views.bytes +
         p->fdk_coef.bytes +
         p->pseudo_coef.bytes + p->pairs.bytes + p->err_flag.bytes;
@@ -873,7 +894,7 @@ YKB_API ykb_status ykb_joseph_fp(ykb_joseph_plan* p, const float* d_volume, floa
     const ykb_volume& v = p->volume;
     if (p->fp_lines.rows > 0) {
         YKB_TRY_CUDA(launch_joseph_fp_lines(d_volume, v.nx, v.ny, v.nz, p->vt.as<float>(),
-            p->views.as<JosephView>(), p->cols.as<float2>(), p->rays.as<float4>(),
+            p->views.as<JosephView>(), p->cols.as<float2>(), p->ray_heights(),
             p->lens.as<float>(), p->n_views, p->nu, p->nv, p->fp_lines, d_proj, accumulate ? 1 : 0, s));
         return YKB_OK;
     }
@@ -1110,10 +1131,10 @@ YKB_API ykb_status ykb_joseph_bp(ykb_joseph_plan* p, const float* d_proj, float*
     DeviceGuard guard(p->device);
     const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     if (p->column_bp)
-        YKB_TRY_CUDA(launch_joseph_bp_lines(d_proj, p->rays.as<float4>(), p->lens.as<float>(),
+        YKB_TRY_CUDA(launch_joseph_bp_lines(d_proj, p->rays.as<float4>(), p->ray_heights(), p->lens.as<float>(),
             p->cols.as<float2>(), p->view_proj.as<float>(), p->views.as<JosephView>(),
-            p->n_views, p->nu, p->nv, p->volume, p->weighted.as<float>(), d_volume,
-            accumulate ? 1 : 0, s));
+            p->n_views, p->nu, p->nv, p->volume, p->bp_runs, p->weighted.as<float>(),
+            p->bp_splits, p->bp_parts, d_volume, accumulate ? 1 : 0, s));
     else
         YKB_TRY_CUDA(launch_joseph_bp(d_proj, p->rays.as<float4>(), p->lens.as<float>(),
             p->view_proj.as<float>(), p->views.as<JosephView>(), p->n_views, p->nu, p->nv,

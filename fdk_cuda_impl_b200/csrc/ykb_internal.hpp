@@ -273,6 +273,16 @@ struct JosephColumnReach {
     double tall = 0.0;             // largest height of a detector row over the source (voxels)
 };
 JosephColumnReach joseph_column_reach(const JosephView& j, int nv, double margin);
+// Whether adjacent rows' rays are less than a voxel apart along z everywhere in
+// the volume (and far enough for FP32 to keep them in order)
+bool joseph_bp_runs(const std::vector<JosephView>& views, int nv);
+// (a2, e2) of the rays, `bytes` from one ray to the next: a table of their own,
+// or without room for it the last two floats of the ray records
+struct JosephHeights {
+    const char* first;
+    int bytes;
+};
+cudaError_t launch_joseph_ray_heights(const float4* rays, long n, float2* out, cudaStream_t s);
 // Forward projection of axial-column scans by detector-column lines
 // (joseph_fp_lines.cu): detector rows of a CTA (0: the lines do not fit, the
 // slab kernel projects) and window of its lines
@@ -288,7 +298,7 @@ inline size_t joseph_line_elems(const ykb_volume& v)
 }
 // vt: joseph_line_elems floats, zeroed once; every call rewrites its interior
 cudaError_t launch_joseph_fp_lines(const float* vol, int nx, int ny, int nz, float* vt,
-    const JosephView* views, const float2* cols, const float4* rays, const float* lens, int n_views,
+    const JosephView* views, const float2* cols, JosephHeights heights, const float* lens, int n_views,
     int nu, int nv, JosephFpLines shape, float* proj, int accumulate, cudaStream_t s);
 cudaError_t launch_joseph_ray_table(const JosephView* views, int n_views,
     int nu, int nv, float4* rays, float* lens, cudaStream_t s);
@@ -311,11 +321,16 @@ cudaError_t launch_siddon_bp(const float* proj, const ykb_cone_view* views, int 
 // then does not apply)
 cudaError_t launch_joseph_column_table(const float4* rays, int n_views, int nu, int nv,
     float2* cols, int* flag, cudaStream_t s);
+// splits of the views of the line backprojector; with more than one its CTAs
+// write FP64 sums to parts[splits][voxels]
+int joseph_bp_splits(const ykb_volume& v, int n_views);
 // matched backprojection for axial-column scans (see launch_joseph_column_table):
-// weighted receives input x chord length per ray
-cudaError_t launch_joseph_bp_lines(const float* proj, const float4* rays, const float* lens,
-    const float2* cols, const float* view_proj, const JosephView* views, int n_views, int nu,
-    int nv, const ykb_volume& vol, float* weighted, float* out, int accumulate, cudaStream_t s);
+// weighted receives input x chord length per ray; runs: adjacent rows' rays are
+// less than a voxel apart along z (joseph_bp_runs)
+cudaError_t launch_joseph_bp_lines(const float* proj, const float4* rays, JosephHeights heights,
+    const float* lens, const float2* cols, const float* view_proj, const JosephView* views, int n_views,
+    int nu, int nv, const ykb_volume& vol, bool runs, float* weighted, int splits, double* parts,
+    float* out, int accumulate, cudaStream_t s);
 cudaError_t launch_joseph_bp(const float* proj, const float4* rays, const float* lens,
     const float* view_proj, const JosephView* views, int n_views, int nu, int nv,
     const ykb_volume& vol, float* weighted, float* out, int accumulate, cudaStream_t s);
@@ -399,12 +414,20 @@ struct ykb_joseph_plan {
     ykb::DeviceBuffer view_proj; // float[n][12]: voxel-space 3x4 projection
     ykb::DeviceBuffer rays;      // float4[n*nv*nu]: (a1, e1, a2, e2)
     ykb::DeviceBuffer lens;      // float[n*nv*nu]: chord length per step
-    // backprojector input x chord length: float[n*nv*nu], or for the column
-    // backprojector float4 (a2, e2, input x chord length, 0)
+    // backprojector input x chord length: float[n*nv*nu]
     ykb::DeviceBuffer weighted;
+    int bp_splits = 1;           // of the line backprojector's views
+    double* bp_parts = nullptr;  // their sums (behind the weighted rays)
+    bool bp_runs = false;        // the line backprojector's lines form in runs
     bool column_bp = false;      // every view's detector columns are axial (line backprojector)
     ykb::DeviceBuffer cols;      // float2[n*nu]: (a1, e1) per detector column
-    ykb::DeviceBuffer slab_y, slab_x;  // transposed volume copies
+    ykb::DeviceBuffer heights;   // float2[n*nv*nu]: (a2, e2), or empty (read from rays)
+    ykb::JosephHeights ray_heights() const
+    {
+        return heights.ptr ? ykb::JosephHeights{heights.as<char>(), 8}
+                           : ykb::JosephHeights{rays.as<char>() + 8, 16};
+    }
+    ykb::DeviceBuffer slab_y, slab_x;  // transposed volume copies (scans without fp_lines)
     ykb::JosephFpLines fp_lines;       // forward projection by lines (column_bp scans)
     ykb::DeviceBuffer vt;              // its volume copy [x][y][z]
     ykb::DeviceBuffer world_views;     // ykb_cone_view[n] (Siddon), uploaded on first use
