@@ -612,16 +612,39 @@ cudaError_t launch_tn(const CUtensorMap* a, const CUtensorMap* t, int nseg, long
 
 } // namespace
 
-int tc_filter_tile_n(int nu)
+namespace {
+
+constexpr int kSms = 148;
+
+// Tile width that filters `rows` rows of nu columns soonest.  The operand feed
+// bounds the tiles (48 KB a K step at 256 columns, 24 at 64, from L2), and every
+// K step of a launch costs its SMs' rounds of tiles: 391 columns run as two tiles
+// of 256 (2 x 48 KB a step) rather than as seven of 64 (7 x 24), although they
+// pad to 512 and 448; 96 columns of few rows as two of 64, side by side.
+// 241 views of 391 x 333 in three calls: 0.61 ms before (tiles of 64), 0.22 now;
+// 60 of 96 x 64: 13.2 and 10.9 us.
+int tile_n(int nu, long rows)
 {
-    // fewest padded columns, then the widest tile
     int best = 0;
-    long best_cols = 0;
+    double best_cost = 0.0;
     for (int tn : {256, 192, 128, 64}) {
-        const long cols = static_cast<long>((nu + tn - 1) / tn) * tn;
-        if (best == 0 || cols < best_cols) { best = tn; best_cols = cols; }
+        const long tiles = (nu + tn - 1) / tn * ((rows + TM - 2) / (TM - 1));
+        const double cost = static_cast<double>((tiles + kSms - 1) / kSms) * (16.0 + tn / 8.0);
+        if (best == 0 || cost < best_cost) { best = tn; best_cost = cost; }
     }
     return best;
+}
+
+} // namespace
+
+int tc_filter_sub_batches(int nu, long rows)
+{
+    // overlapping the preweight pays while each sub-batch still fills the GPU
+    // with two rounds of tiles (180 views of 192 x 128, 182 tiles: filter stage
+    // 90 us in four sub-batches of 46 tiles, 50 in one)
+    const int tn = tile_n(nu, rows);
+    const long tiles = (nu + tn - 1) / tn * ((rows + TM - 2) / (TM - 1));
+    return static_cast<int>(std::min<long>(std::max<long>(tiles / (2 * kSms), 1), 4));
 }
 
 bool tcgen05_filter_supported(int nu) { return tma_encode() != nullptr && nu >= 16; }
@@ -664,7 +687,7 @@ cudaError_t launch_fdk_ramp_tcgen05(const __nv_bfloat16* const a_parts[3],
     int nv, float* out, int layout, int ldc, int near_chunks, int* err, cudaStream_t s)
 {
     if (rows <= 0) return cudaSuccess;
-    const int tn = tc_filter_tile_n(nu);
+    const int tn = tile_n(nu, rows);
     const int nparts = a_parts[2] && t_parts[2] ? 3 : 2;
     CUtensorMap a[3], t[3];
     // A: [rows][ld] K-major, box 64 x 128; T: [nu][ld] K-major, box 64 x TN

@@ -367,8 +367,8 @@ ykb_status filter_chunk_(ykb_fdk_plan* p, const void* proj, int proj_dtype, int 
         // sub-batches of views: the preweight (memory bound) of sub-batch
         // b + 1 runs on the auxiliary stream under the ramp filter (tensor
         // bound) of sub-batch b
-        constexpr int kSub = ykb_fdk_plan::kFilterSubBatches;
-        const int nsub = count >= 16 * kSub ? kSub : 1;
+        const int nsub = std::min(tc_filter_sub_batches(p->nu, static_cast<long>(count) * p->nv), count);
+        static_assert(ykb_fdk_plan::kFilterSubBatches == 4, "events for every sub-batch");
         if (nsub > 1 && !p->aux_stream) {
             YKB_TRY_CUDA(cudaStreamCreateWithFlags(&p->aux_stream, cudaStreamNonBlocking));
             YKB_TRY_CUDA(cudaEventCreateWithFlags(&p->aux_in, cudaEventDisableTiming));

@@ -208,6 +208,9 @@ cudaError_t launch_fdk_ramp_tcgen05(const __nv_bfloat16* const a_parts[3],
     int* err_flag, cudaStream_t s);
 int tc_filter_near_chunks(const std::vector<double>& h, int nu);
 bool tcgen05_filter_supported(int nu);
+// view sub-batches (1 to 4) in which the preweight of one runs under the filter
+// of the one before
+int tc_filter_sub_batches(int nu, long rows);
 int tc_filter_lda(int nu);
 cudaError_t launch_fdk_backproject(const void* filtered, int dtype,
     const FdkViewCoef* coef, int n_views, int nu, int nv, int ld,
