@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(128) joseph_fp_padded_kernel(const float* __re
         kMagicBits * static_cast<uint32_t>(p1 + 1);
     const uint32_t last = static_cast<uint32_t>(plane) - static_cast<uint32_t>(p1) - 2u;
     const f2 A = f2pack(r.a1, r.a2), E = f2pack(r.e1, r.e2);
-    const f2 H = f2pack(0.5f, 0.5f), M = f2pack(kMagic, kMagic);
+    const f2 M = f2pack(kMagic, kMagic);
     float c0 = static_cast<float>(wlo) - 0.5f * (j.n0 - 1);  // exact: integers and halves
     // FP64 ray sum: keeps the adjoint identity at the 1e-7 level even where
     // <Ax, y> cancels to 1e-4 of its terms
@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(128) joseph_fp_padded_kernel(const float* __re
         // a slice outside this lane's range reads the zero border corner
         const bool in = sq >= lo && sq <= hi;
         const f2 f = f2fma(A, f2pack(c0, c0), E);
-        const f2 t = f2add(f2sub(f, H), M);
+        const f2 t = f2add_rm(f, M);
         float t1, t2, w1, w2;
         f2unpack(t, t1, t2);
         f2unpack(f2sub(f, f2sub(t, M)), w1, w2);
@@ -349,7 +349,7 @@ __global__ void joseph_weight_rays_kernel(const float* __restrict__ proj,
 // f < 1/2 may differ, by one rounding of a weight below 1/2.
 __device__ __forceinline__ float hat_weight(float f, float jf)
 {
-    return fmaxf(0.f, 1.f - fabsf(f - jf));
+    return __saturatef(1.f - fabsf(f - jf));  // at most 1: one add with saturation
 }
 
 // Detector box of the slice rectangle [j1lo - 1, j1hi + 1] x [j2lo - 1,
