@@ -775,6 +775,10 @@ __global__ void __launch_bounds__(kLineThreads, 3) joseph_bp_lines_kernel(
 //   * the last warp, which the lines rarely reach, prepares the next view's
 //     boxes, and every thread has its next line's first rays in flight while it
 //     sums its column: two barriers a view.
+// Bound: instruction issue and the shared-memory data path together (55 and 66 %;
+// three wavefronts a request in the column sums), with 24 warps an SM.  256^3 x
+// 360 x 384^2: 21.3 ms, before 24.9; the runs alone, without the last two points:
+// 25.2; (a2, e2) from the 16-byte ray records instead of a table of their own: 22.2.
 // ---------------------------------------------------------------------------
 constexpr int kRunGroup = 4;  // rays of a line loaded together
 

@@ -55,3 +55,33 @@ def test_line_projector_matches_slab_projector(oracle, cuda_device, monkeypatch,
         assert K.rel_rmse(a.cpu().numpy(), ref) <= 1e-5
     lines.close()
     slabs.close()
+
+
+@pytest.mark.parametrize("case", CASES + [(90, 50, 40, 1.7, 1.7, (34, 35, 33), (1.0, 1.0, 1.0), False)])
+def test_line_backprojector_matches_gather(oracle, cuda_device, monkeypatch, case):
+    # lines formed in runs (rows closer than a voxel) or by splatting, and views
+    # split over CTAs for volumes of few blocks; the voxel gather applies the
+    # same weights: two FP32 summation orders of at most a few hundred terms
+    import torch
+    from fdk_cuda_impl_b200.projectors import JosephPlan
+    views, nu, nv, pu, pv, n, vox, flipped = case
+    scan = CircularScan(views, views, 500.0, 1000.0, nu, nv, pu, pv, start_angle_rad=0.05)
+    grid = VolumeGrid(*n, vox, (0.4, -0.7, 0.2))
+    table = scan.views()
+    if flipped:
+        table["detS"][:, :3] += (nv - 1) * table["detV"][:, :3]
+        table["detV"][:, :3] *= -1
+    y = torch.from_numpy(oracle.normal((views, nv, nu), 7)).cuda()
+    lines = JosephPlan(table, nu, nv, grid)
+    monkeypatch.setenv("YKB_JOSEPH_BP", "gather")
+    gather = JosephPlan(table, nu, nv, grid)
+    a, b = lines.adjoint(y), gather.adjoint(y)
+    assert torch.isfinite(a).all() and float(b.abs().max()) > 0
+    assert K.rel_rmse(a.cpu().numpy(), b.cpu().numpy()) <= 1e-6
+    assert torch.equal(lines.adjoint(y), a)
+    both = lines.adjoint(y, b.clone(), accumulate=True)
+    assert K.rel_rmse(both.cpu().numpy(), 2 * b.cpu().numpy()) <= 1e-6
+    # where no ray passes both are exactly zero
+    assert torch.equal(lines.adjoint(torch.zeros_like(y)), torch.zeros_like(b))
+    lines.close()
+    gather.close()
