@@ -412,14 +412,20 @@ JosephFpLines joseph_fp_lines_shape(const std::vector<JosephView>& views, int nv
     return best;
 }
 
+cudaError_t launch_joseph_line_volume(const float* vol, int nx, int ny, int nz, float* vt, cudaStream_t s)
+{
+    const int nzp = joseph_line_pitch(nz);
+    transpose_xyz_kernel<<<dim3((nx + 31) / 32, (nzp + 31) / 32, ny), dim3(32, 8), 0, s>>>(vol, nx, ny,
+        nz, nzp, vt);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_joseph_fp_lines(const float* vol, int nx, int ny, int nz, float* vt,
     const JosephView* views, const float2* cols, JosephHeights heights, const float* lens, int n_views,
     int nu, int nv, JosephFpLines shape, float* proj, int accumulate, cudaStream_t s)
 {
     const int nzp = joseph_line_pitch(nz);
-    transpose_xyz_kernel<<<dim3((nx + 31) / 32, (nzp + 31) / 32, ny), dim3(32, 8), 0, s>>>(vol, nx, ny,
-        nz, nzp, vt);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_joseph_line_volume(vol, nx, ny, nz, vt, s);
     for (int done = 0; e == cudaSuccess && done < n_views; done += 65535) {
         const dim3 grid((nu + kCols - 1) / kCols, (nv + shape.rows - 1) / shape.rows,
             std::min(n_views - done, 65535));

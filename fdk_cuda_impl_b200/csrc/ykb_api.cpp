@@ -878,7 +878,7 @@ YKB_API size_t ykb_joseph_workspace_bytes(const ykb_joseph_plan* p)
     if (!p) return 0;
     return p->views.bytes + p->view_proj.bytes + p->rays.bytes + p->lens.bytes +
         p->weighted.bytes + p->cols.bytes + p->heights.bytes + p->vt.bytes + p->slab_x.bytes + p->slab_y.bytes +
-        p->world_views.bytes +
+        p->world_views.bytes + p->siddon_vt.bytes +
         p->fdk_coef.bytes +
         p->pseudo_coef.bytes + p->pairs.bytes + p->err_flag.bytes;
 }
@@ -984,9 +984,26 @@ ykb_status pseudo_bp(ykb_joseph_plan* p, const float* d_proj, float* d_volume, i
     return YKB_OK;
 }
 
+// The volume copy of the Siddon pair by detector columns; without room for it
+// the rays are walked one by one.
+ykb_status prepare_siddon_lines(ykb_joseph_plan* p, const VolumeGrid& g, cudaStream_t s)
+{
+    p->siddon_lines = 0;
+    if (!siddon_lines_apply(p->cone_views.data(), p->n_views, p->nv, g)) return YKB_OK;
+    if (p->siddon_vt.alloc(2 * sizeof(float) * joseph_line_elems(p->volume)) != cudaSuccess) {
+        cudaGetLastError();
+        return YKB_OK;
+    }
+    YKB_TRY_CUDA(cudaEventCreateWithFlags(&p->siddon_done, cudaEventDisableTiming));
+    YKB_TRY_CUDA(cudaMemsetAsync(p->siddon_vt.ptr, 0, p->siddon_vt.bytes, s));
+    p->siddon_lines = 1;
+    return YKB_OK;
+}
+
 ykb_status siddon(ykb_joseph_plan* p, bool forward, const float* d_in, float* d_out,
     int accumulate, cudaStream_t s)
 {
+    const std::lock_guard<std::mutex> lock(p->siddon_mutex);
     if (!p->world_views.ptr) {
         const size_t bytes = sizeof(ykb_cone_view) * p->cone_views.size();
         cudaError_t e = p->world_views.alloc(bytes);
@@ -1000,10 +1017,26 @@ ykb_status siddon(ykb_joseph_plan* p, bool forward, const float* d_in, float* d_
     }
     const VolumeGrid g = make_grid(p->volume);
     const ykb_cone_view* v = p->world_views.as<ykb_cone_view>();
+    if (p->siddon_lines < 0)
+        if (const ykb_status st = prepare_siddon_lines(p, g, s)) return st;
+    if (p->siddon_lines == 0) {
+        if (forward)
+            YKB_TRY_CUDA(launch_siddon_fp(d_in, v, p->n_views, p->nu, p->nv, g, d_out, accumulate, s));
+        else
+            YKB_TRY_CUDA(launch_siddon_bp(d_in, v, p->n_views, p->nu, p->nv, g, d_out, accumulate, s));
+        return YKB_OK;
+    }
+    // a captured call is ordered by its graph
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    YKB_TRY_CUDA(cudaStreamIsCapturing(s, &capture));
+    const bool ordered = capture == cudaStreamCaptureStatusNone;
+    if (ordered) YKB_TRY_CUDA(cudaStreamWaitEvent(s, p->siddon_done, 0));
+    float* vt = p->siddon_vt.as<float>();
     if (forward)
-        YKB_TRY_CUDA(launch_siddon_fp(d_in, v, p->n_views, p->nu, p->nv, g, d_out, accumulate, s));
+        YKB_TRY_CUDA(launch_siddon_fp_lines(d_in, vt, v, p->n_views, p->nu, p->nv, g, d_out, accumulate, s));
     else
-        YKB_TRY_CUDA(launch_siddon_bp(d_in, v, p->n_views, p->nu, p->nv, g, d_out, accumulate, s));
+        YKB_TRY_CUDA(launch_siddon_bp_lines(d_in, vt, v, p->n_views, p->nu, p->nv, g, d_out, accumulate, s));
+    if (ordered) YKB_TRY_CUDA(cudaEventRecord(p->siddon_done, s));
     return YKB_OK;
 }
 

@@ -7,6 +7,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -299,6 +300,7 @@ inline size_t joseph_line_elems(const ykb_volume& v)
 {
     return static_cast<size_t>(v.nx + 2 * kLinePad) * (v.ny + 2 * kLinePad) * joseph_line_pitch(v.nz);
 }
+cudaError_t launch_joseph_line_volume(const float* vol, int nx, int ny, int nz, float* vt, cudaStream_t s);
 // vt: joseph_line_elems floats, zeroed once; every call rewrites its interior
 cudaError_t launch_joseph_fp_lines(const float* vol, int nx, int ny, int nz, float* vt,
     const JosephView* views, const float2* cols, JosephHeights heights, const float* lens, int n_views,
@@ -319,6 +321,15 @@ cudaError_t launch_siddon_fp(const float* vol, const ykb_cone_view* views, int n
     int nv, const VolumeGrid& g, float* proj, int accumulate, cudaStream_t s);
 cudaError_t launch_siddon_bp(const float* proj, const ykb_cone_view* views, int n_views, int nu,
     int nv, const VolumeGrid& g, float* vol, int accumulate, cudaStream_t s);
+// The same pair for axial-column scans by detector columns, over the volume copy
+// of joseph_line_elems floats (see launch_joseph_line_volume); the backprojector
+// sums even and odd views in a copy each: half the additions to a voxel, to sums
+// half as large, so half their rounding
+bool siddon_lines_apply(const ykb_cone_view* views, int n_views, int nv, const VolumeGrid& g);
+cudaError_t launch_siddon_fp_lines(const float* vol, float* vt, const ykb_cone_view* views, int n_views,
+    int nu, int nv, const VolumeGrid& g, float* proj, int accumulate, cudaStream_t s);
+cudaError_t launch_siddon_bp_lines(const float* proj, float* vt, const ykb_cone_view* views, int n_views,
+    int nu, int nv, const VolumeGrid& g, float* vol, int accumulate, cudaStream_t s);
 // (a1, e1) of every detector column from its first row into cols[n][nu];
 // flag[0] = 1 when any ray of a column differs (the line backprojector
 // then does not apply)
@@ -433,7 +444,14 @@ struct ykb_joseph_plan {
     ykb::DeviceBuffer slab_y, slab_x;  // transposed volume copies (scans without fp_lines)
     ykb::JosephFpLines fp_lines;       // forward projection by lines (column_bp scans)
     ykb::DeviceBuffer vt;              // its volume copy [x][y][z]
-    ykb::DeviceBuffer world_views;     // ykb_cone_view[n] (Siddon), uploaded on first use
+    // Siddon, set up on first use: the views, and for axial-column scans a volume
+    // copy.  Calls on different streams take turns on the copy
+    ykb::DeviceBuffer world_views;     // ykb_cone_view[n]
+    int siddon_lines = -1;             // by detector columns: 1, ray by ray: 0, undecided: -1
+    ykb::DeviceBuffer siddon_vt;
+    cudaEvent_t siddon_done = nullptr; // the last call's work on the copy
+    std::mutex siddon_mutex;
+    ~ykb_joseph_plan() { if (siddon_done) cudaEventDestroy(siddon_done); }
     // pseudo-matched backprojection, set up on first use
     bool pseudo_ready = false;
     bool pseudo_axial = false;         // untilted detector: the axial column walk
