@@ -777,8 +777,9 @@ __global__ void __launch_bounds__(kLineThreads, 3) joseph_bp_lines_kernel(
 //     sums its column: two barriers a view.
 // Bound: instruction issue and the shared-memory data path together (55 and 66 %;
 // three wavefronts a request in the column sums), with 24 warps an SM.  256^3 x
-// 360 x 384^2: 21.3 ms, before 24.9; the runs alone, without the last two points:
-// 25.2; (a2, e2) from the 16-byte ray records instead of a table of their own: 22.2.
+// 360 x 384^2: 21.1 ms, before 24.9; the runs alone, without the last two points:
+// 25.2; (a2, e2) from the 16-byte ray records instead of a table of their own: 22.2;
+// two sets of rays in turn instead of a copy of the set in flight: 22.1 (spills).
 // ---------------------------------------------------------------------------
 constexpr int kRunGroup = 4;  // rays of a line loaded together
 
@@ -846,13 +847,14 @@ __device__ __forceinline__ void prepare_run_view(RunView& out, const ViewProj& m
     if (lane == 0) out.passes = (most + kLineMax - 1) / kLineMax;
 }
 
-// a thread's line: its first ray, step to the next, number of rays, pair and
-// column (count 0: none)
+// a thread's line: byte offsets of its first ray in the view's (a2, e2) and
+// values, steps to the next ray, number of rays (0: none), pair and column
 struct RunLine {
-    int first, step, count, pair, column;
+    uint32_t at_a, at_v, step_a, step_v;
+    int count, pair, column;
 };
 
-__device__ __forceinline__ RunLine run_line(const RunView& rv, int pass, bool up, int nu)
+__device__ __forceinline__ RunLine run_line(const RunView& rv, int pass, bool up, int nu, int ray_bytes)
 {
     constexpr int P = kLineBlock / 2;
     RunLine l;
@@ -876,8 +878,13 @@ __device__ __forceinline__ RunLine run_line(const RunView& rv, int pass, bool up
     l.pair = pair;
     l.column = c;
     l.count = c < kLineMax && iu <= b.y ? b.w - b.z + 1 : 0;
-    l.first = (up ? b.z : b.w) * nu + iu;
-    l.step = up ? nu : -nu;
+    // in the order of increasing f2
+    const uint32_t first = static_cast<uint32_t>((up ? b.z : b.w) * nu + iu);
+    const uint32_t step = up ? static_cast<uint32_t>(nu) : 0u - static_cast<uint32_t>(nu);
+    l.at_a = first * static_cast<uint32_t>(ray_bytes);
+    l.step_a = step * static_cast<uint32_t>(ray_bytes);
+    l.at_v = first * 4u;
+    l.step_v = step * 4u;
     return l;
 }
 
@@ -886,18 +893,61 @@ struct RunRays {
     float v[kRunGroup];
 };
 
-// rays i .. i + 3 of a line; past its last ray, that one with value zero
-__device__ __forceinline__ void load_rays(RunRays& r, const char* rays, int ray_bytes, const float* wv,
-    const RunLine& l, int i)
+// the line's next four rays; of the last `left` < 4, the last one is repeated
+// with value zero
+__device__ __forceinline__ void load_rays(RunRays& r, const char* rays, const char* wv, RunLine& l, int left)
 {
+    if (left >= kRunGroup) {
 #pragma unroll
-    for (int q = 0; q < kRunGroup; ++q) {
-        const bool in = i + q < l.count;
-        const int at = l.first + (in ? i + q : l.count - 1) * l.step;
-        r.a[q] = __ldg(reinterpret_cast<const float2*>(rays + static_cast<long>(at) * ray_bytes));
-        r.v[q] = in ? __ldg(wv + at) : 0.f;
+        for (int q = 0; q < kRunGroup; ++q) {
+            r.a[q] = __ldg(reinterpret_cast<const float2*>(rays + l.at_a));
+            r.v[q] = __ldg(reinterpret_cast<const float*>(wv + l.at_v));
+            l.at_a += l.step_a;
+            l.at_v += l.step_v;
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < kRunGroup; ++q) {
+            r.a[q] = __ldg(reinterpret_cast<const float2*>(rays + l.at_a));
+            r.v[q] = q < left ? __ldg(reinterpret_cast<const float*>(wv + l.at_v)) : 0.f;
+            if (q + 1 < left) {
+                l.at_a += l.step_a;
+                l.at_v += l.step_v;
+            }
+        }
     }
 }
+
+// A column's two sums on each of two adjacent slices csa, csb as its rays go by.
+template <int ZC>
+struct RunSums {
+    float cur[2], lo[2], hi[2];
+    __device__ __forceinline__ void add(const RunRays& r, float csa, float csb, uint32_t slot0, float* La,
+        float* Lb)
+    {
+        const f2 M = f2pack(kMagic, kMagic);
+#pragma unroll
+        for (int q = 0; q < kRunGroup; ++q) {
+            const f2 f = f2pack(fmaf(r.a[q].x, csa, r.a[q].y), fmaf(r.a[q].x, csb, r.a[q].y));
+            const f2 t = f2add_rm(f, M);
+            const f2 vv = f2pack(r.v[q], r.v[q]), u = f2mul(vv, f2sub(f, f2sub(t, M)));
+            float tt[2], uu[2], xx[2];
+            f2unpack(t, tt[0], tt[1]);
+            f2unpack(u, uu[0], uu[1]);
+            f2unpack(f2sub(vv, u), xx[0], xx[1]);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const bool begins = tt[e] != cur[e];  // the next voxel
+                lo[e] = (begins ? hi[e] : lo[e]) + xx[e];
+                hi[e] = (begins ? 0.f : hi[e]) + uu[e];
+                cur[e] = tt[e];
+                // slot ZC + 1 takes what falls outside
+                const uint32_t slot = min(__float_as_uint(tt[e]) - slot0, static_cast<uint32_t>(ZC + 1));
+                (e ? Lb : La)[slot * kLineMax] = lo[e];
+            }
+        }
+    }
+};
 
 template <int ZC>
 __global__ void __launch_bounds__(kLineThreads, 3) joseph_bp_runs_kernel(
@@ -926,25 +976,24 @@ __global__ void __launch_bounds__(kLineThreads, 3) joseph_bp_runs_kernel(
     for (int q = 0; q < ZC; ++q) total[q * kLineThreads + tid] = 0.0;
     // slot of floor(f2) + 1 from the floor word of f2 (wrapping)
     const uint32_t slot0 = kMagicBits + static_cast<uint32_t>(z0 - 1);
-    const f2 M = f2pack(kMagic, kMagic);
     float acc[ZC];  // FP32 over sixteen views, then into the FP64 sums
 #pragma unroll
     for (int q = 0; q < ZC; ++q) acc[q] = 0.f;
     if (warp == kLast) prepare_run_view<ZC>(rviews[k0 & 1], vp[k0], views[k0], X0, Y0, z0, nu, nv);
     __syncthreads();
-    RunLine line = run_line(rviews[k0 & 1], 0, views[k0].detV[2] > 0.0, nu);
+    RunLine line = run_line(rviews[k0 & 1], 0, views[k0].detV[2] > 0.0, nu, ray_bytes);
     RunRays next;
-    if (line.count > 0)
-        load_rays(next, rays + static_cast<long>(k0) * view_rays * ray_bytes, ray_bytes,
-            wv + static_cast<long>(k0) * view_rays, line, 0);
+    const char* const values = reinterpret_cast<const char*>(wv);
+    const long view_a = static_cast<long>(view_rays) * ray_bytes, view_v = static_cast<long>(view_rays) * 4;
+    if (line.count > 0) load_rays(next, rays + k0 * view_a, values + k0 * view_v, line, line.count);
     for (int k = k0; k < k1; ++k) {
         const JosephView& j = views[k];
         const RunView& rv = rviews[k & 1];
         const bool ax0 = j.axis == 0;
         const int S0 = ax0 ? X0 : Y0;
         const float half = 0.5f * (j.n0 - 1);
-        const char* rk = rays + static_cast<long>(k) * view_rays * ray_bytes;
-        const float* wk = wv + static_cast<long>(k) * view_rays;
+        const char* const rk = rays + k * view_a;
+        const char* const wk = values + k * view_v;
         const int passes = rv.passes;
         const bool up = j.detV[2] > 0.0;  // f2 grows with the row
         // this thread's voxel column: its slice, minor-1 index, candidates
@@ -955,8 +1004,8 @@ __global__ void __launch_bounds__(kLineThreads, 3) joseph_bp_runs_kernel(
         if (mine) column_span(vp[k], j, c0, j1, nu, cu0, cu1);
         for (int pass = 0; pass < max(passes, 1); ++pass) {
             if (pass > 0) {
-                line = run_line(rv, pass, up, nu);
-                if (line.count > 0) load_rays(next, rk, ray_bytes, wk, line, 0);
+                line = run_line(rv, pass, up, nu, ray_bytes);
+                if (line.count > 0) load_rays(next, rk, wk, line, line.count);
             }
             // ---- this thread's line, on both slices of its pair
             if (line.count > 0) {
@@ -971,42 +1020,25 @@ __global__ void __launch_bounds__(kLineThreads, 3) joseph_bp_runs_kernel(
                     at[0] = fmaf(ce.x, csa, ce.y);
                     at[LM] = fmaf(ce.x, csb, ce.y);
                 }
-                float cur[2], lo[2] = {0.f, 0.f}, hi[2] = {0.f, 0.f};
-                cur[0] = __fadd_rd(fmaf(next.a[0].x, csa, next.a[0].y), kMagic);
-                cur[1] = __fadd_rd(fmaf(next.a[0].x, csb, next.a[0].y), kMagic);
-                const int start[2] = {static_cast<int>(__float_as_uint(cur[0]) - slot0),
-                                      static_cast<int>(__float_as_uint(cur[1]) - slot0)};
-                for (int i = 0; i < line.count; i += kRunGroup) {
+                RunSums<ZC> sums;
+                sums.cur[0] = __fadd_rd(fmaf(next.a[0].x, csa, next.a[0].y), kMagic);
+                sums.cur[1] = __fadd_rd(fmaf(next.a[0].x, csb, next.a[0].y), kMagic);
+                sums.lo[0] = sums.lo[1] = sums.hi[0] = sums.hi[1] = 0.f;
+                const int start[2] = {static_cast<int>(__float_as_uint(sums.cur[0]) - slot0),
+                                      static_cast<int>(__float_as_uint(sums.cur[1]) - slot0)};
+                // four rays while the next four are in flight
+                for (int left = line.count - kRunGroup; ; left -= kRunGroup) {
                     const RunRays r = next;
-                    if (i + kRunGroup < line.count) load_rays(next, rk, ray_bytes, wk, line, i + kRunGroup);
-#pragma unroll
-                    for (int q = 0; q < kRunGroup; ++q) {
-                        const f2 f = f2pack(fmaf(r.a[q].x, csa, r.a[q].y), fmaf(r.a[q].x, csb, r.a[q].y));
-                        const f2 t = f2add_rm(f, M);
-                        const f2 vv = f2pack(r.v[q], r.v[q]), u = f2mul(vv, f2sub(f, f2sub(t, M)));
-                        float tt[2], uu[2], xx[2];
-                        f2unpack(t, tt[0], tt[1]);
-                        f2unpack(u, uu[0], uu[1]);
-                        f2unpack(f2sub(vv, u), xx[0], xx[1]);
-#pragma unroll
-                        for (int e = 0; e < 2; ++e) {
-                            const bool begins = tt[e] != cur[e];  // the next voxel
-                            lo[e] = (begins ? hi[e] : lo[e]) + xx[e];
-                            hi[e] = (begins ? 0.f : hi[e]) + uu[e];
-                            cur[e] = tt[e];
-                            // slot ZC + 1 takes what falls outside
-                            const uint32_t slot = min(__float_as_uint(tt[e]) - slot0,
-                                static_cast<uint32_t>(ZC + 1));
-                            (e ? Lb : La)[slot * LM] = lo[e];
-                        }
-                    }
+                    if (left > 0) load_rays(next, rk, wk, line, left);
+                    sums.add(r, csa, csb, slot0, La, Lb);
+                    if (left <= 0) break;
                 }
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     // the entry after the last ray's; entries no ray reaches are zero
                     float* const L = e ? Lb : La;
-                    const int last = static_cast<int>(__float_as_uint(cur[e]) - slot0);
-                    if (last >= 0 && last < ZC) L[(last + 1) * LM] = hi[e];
+                    const int last = static_cast<int>(__float_as_uint(sums.cur[e]) - slot0);
+                    if (last >= 0 && last < ZC) L[(last + 1) * LM] = sums.hi[e];
                     for (int q = min(start[e] - 1, ZC); q >= 1; --q) L[q * LM] = 0.f;
                     for (int q = max(last + 2, 1); q <= ZC; ++q) L[q * LM] = 0.f;
                 }
@@ -1018,10 +1050,8 @@ __global__ void __launch_bounds__(kLineThreads, 3) joseph_bp_runs_kernel(
             __syncthreads();
             // the next view's first rays, in flight during the sums
             if (pass + 1 >= passes && k + 1 < k1) {
-                line = run_line(rviews[(k + 1) & 1], 0, views[k + 1].detV[2] > 0.0, nu);
-                if (line.count > 0) 
-                    load_rays(next, rk + static_cast<long>(view_rays) * ray_bytes, ray_bytes,
-                        wk + view_rays, line, 0);
+                line = run_line(rviews[(k + 1) & 1], 0, views[k + 1].detV[2] > 0.0, nu, ray_bytes);
+                if (line.count > 0) load_rays(next, rk + view_a, wk + view_v, line, line.count);
             }
             // ---- this column: its candidates among this pass's lines
             if (mine) {
