@@ -282,7 +282,14 @@ YKB_API ykb_status ykb_fdk_plan_create_ex(const ykb_cone_view* views, int n_view
     // workspace with the filter that it did not read before
     p->filtered_floats = static_cast<size_t>(p->batch_capacity) * filtered_view_floats(p);
     p->part_floats = p->layout == kFilteredPairs ? fdk_tma_part_floats(make_grid(p->volume), n_views) : 0;
-    if ((e = p->work_filtered.alloc(sizeof(float) * (p->filtered_floats + p->part_floats))) != cudaSuccess) {
+    e = p->work_filtered.alloc(sizeof(float) * (p->filtered_floats + p->part_floats));
+    if (e != cudaSuccess && p->part_floats > 0) {
+        // without room for them the views are not split
+        cudaGetLastError();
+        p->part_floats = 0;
+        e = p->work_filtered.alloc(sizeof(float) * p->filtered_floats);
+    }
+    if (e != cudaSuccess) {
         delete p;
         return cuda_status(e, "cudaMalloc (FDK filtered workspace)");
     }
@@ -809,20 +816,23 @@ YKB_API ykb_status ykb_joseph_plan_create(const ykb_cone_view* views, int n_view
     if (const char* env = std::getenv("YKB_JOSEPH_BP"))
         if (std::strcmp(env, "gather") == 0) columns = false;
     if (e == cudaSuccess && columns) {
-        DeviceBuffer flag;
         int differs = 1;
-        if ((e = p->cols.alloc(sizeof(float2) * n_views * nu)) == cudaSuccess &&
-            (e = flag.alloc(sizeof(int))) == cudaSuccess &&
-            (e = launch_joseph_column_table(p->rays.as<float4>(), n_views, nu, nv,
-                 p->cols.as<float2>(), flag.as<int>(), s)) == cudaSuccess &&
-            (e = cudaMemcpyAsync(&differs, flag.ptr, sizeof(int), cudaMemcpyDeviceToHost, s)) ==
-                cudaSuccess)
-            e = cudaStreamSynchronize(s);
+        // the check's flag lies behind the column table
+        const size_t cols = static_cast<size_t>(n_views) * nu;
+        if ((e = p->cols.alloc(sizeof(float2) * (cols + 1))) == cudaSuccess) {
+            int* const flag = reinterpret_cast<int*>(p->cols.as<float2>() + cols);
+            if ((e = launch_joseph_column_table(p->rays.as<float4>(), n_views, nu, nv,
+                     p->cols.as<float2>(), flag, s)) == cudaSuccess &&
+                (e = cudaMemcpyAsync(&differs, flag, sizeof(int), cudaMemcpyDeviceToHost, s)) ==
+                    cudaSuccess)
+                e = cudaStreamSynchronize(s);
+        }
         p->column_bp = e == cudaSuccess && differs == 0;
         if (!p->column_bp) p->cols.reset();
         if (p->column_bp) {
             p->fp_lines = joseph_fp_lines_shape(p->host_views, nv);
-            p->bp_runs = joseph_bp_runs(p->host_views, nv);
+            // (32-bit byte offsets of a view's ray records)
+            p->bp_runs = static_cast<long>(nu) * nv < (1L << 27) && joseph_bp_runs(p->host_views, nv);
             // without room for the table the ray records serve
             if (p->heights.alloc(sizeof(float2) * rays) == cudaSuccess)
                 e = launch_joseph_ray_heights(p->rays.as<float4>(), static_cast<long>(rays),
@@ -949,11 +959,17 @@ ykb_status prepare_pseudo(ykb_joseph_plan* p, cudaStream_t s)
             const int ld = (p->nu + 1) / 2 * 2;
             const size_t part_floats = fdk_tma_part_floats(make_grid(p->volume), p->n_views);
             const size_t pair_floats = static_cast<size_t>(p->n_views) * (p->nv + 1) * ld * 2;
-            if (p->pairs.alloc(sizeof(float) * (pair_floats + part_floats)) == cudaSuccess) {
-                p->pseudo_box = box;
-                p->pseudo_ld = ld;
+            const bool split = part_floats > 0 &&
+                p->pairs.alloc(sizeof(float) * (pair_floats + part_floats)) == cudaSuccess;
+            if (split) {
                 p->pseudo_parts = p->pairs.as<float>() + pair_floats;
                 p->pseudo_part_floats = part_floats;
+            } else if (part_floats > 0) {
+                cudaGetLastError();  // without room for their sums the views are not split
+            }
+            if (split || p->pairs.alloc(sizeof(float) * pair_floats) == cudaSuccess) {
+                p->pseudo_box = box;
+                p->pseudo_ld = ld;
             } else {
                 // without room for the staged pairs the bounds-checked kernel runs
                 cudaGetLastError();
