@@ -1035,24 +1035,24 @@ ykb_status siddon(ykb_joseph_plan* p, bool forward, const float* d_in, float* d_
     const ykb_cone_view* v = p->world_views.as<ykb_cone_view>();
     if (p->siddon_lines < 0)
         if (const ykb_status st = prepare_siddon_lines(p, g, s)) return st;
-    if (p->siddon_lines == 0) {
+    // a graph may be replayed beside other calls of the plan, which no event
+    // orders then: a captured call takes the walk, which shares no workspace
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    YKB_TRY_CUDA(cudaStreamIsCapturing(s, &capture));
+    if (p->siddon_lines == 0 || capture != cudaStreamCaptureStatusNone) {
         if (forward)
             YKB_TRY_CUDA(launch_siddon_fp(d_in, v, p->n_views, p->nu, p->nv, g, d_out, accumulate, s));
         else
             YKB_TRY_CUDA(launch_siddon_bp(d_in, v, p->n_views, p->nu, p->nv, g, d_out, accumulate, s));
         return YKB_OK;
     }
-    // a captured call is ordered by its graph
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    YKB_TRY_CUDA(cudaStreamIsCapturing(s, &capture));
-    const bool ordered = capture == cudaStreamCaptureStatusNone;
-    if (ordered) YKB_TRY_CUDA(cudaStreamWaitEvent(s, p->siddon_done, 0));
+    YKB_TRY_CUDA(cudaStreamWaitEvent(s, p->siddon_done, 0));
     float* vt = p->siddon_vt.as<float>();
     if (forward)
         YKB_TRY_CUDA(launch_siddon_fp_lines(d_in, vt, v, p->n_views, p->nu, p->nv, g, d_out, accumulate, s));
     else
         YKB_TRY_CUDA(launch_siddon_bp_lines(d_in, vt, v, p->n_views, p->nu, p->nv, g, d_out, accumulate, s));
-    if (ordered) YKB_TRY_CUDA(cudaEventRecord(p->siddon_done, s));
+    YKB_TRY_CUDA(cudaEventRecord(p->siddon_done, s));
     return YKB_OK;
 }
 

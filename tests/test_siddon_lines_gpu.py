@@ -55,6 +55,14 @@ def test_siddon_pair_matches_oracle(oracle, cuda_device, case):
     torch.cuda.synchronize()
     for i, o in enumerate(out):
         assert K.rel_rmse(o.cpu().numpy(), ref_fp if i % 3 else ref_bp) <= 1e-5
+    # a captured call
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        gp, gb = plan.forward_siddon(xd), plan.backproject_siddon(yd)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert K.rel_rmse(gp.cpu().numpy(), ref_fp) <= 1e-5
+    assert K.rel_rmse(gb.cpu().numpy(), ref_bp) <= 1e-5
     # a voxel that no ray of a missing column reads does not leak into it
     if n[0] > 20:
         bad = xd.clone()
