@@ -371,8 +371,10 @@ __device__ __forceinline__ void footprint_box_range(const ViewProj& m, const Jos
         else if (j.axis == 1) { px = q1; py = c0; pz = q2; }
         else { px = q1; py = q2; pz = c0; }
         const float w = fmaf(m.m[8], px, fmaf(m.m[9], py, fmaf(m.m[10], pz, m.m[11])));
-        // the box only needs a few 1e-6 px: correctly rounded reciprocal
-        const float rw = __frcp_rn(w);
+        // one ulp of the reciprocal moves a corner by less than the margin below
+        // column 400000
+        float rw;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rw) : "f"(w));
         const float u = fmaf(m.m[0], px, fmaf(m.m[1], py, fmaf(m.m[2], pz, m.m[3]))) * rw;
         const float v = fmaf(m.m[4], px, fmaf(m.m[5], py, fmaf(m.m[6], pz, m.m[7]))) * rw;
         umin = fminf(umin, u); umax = fmaxf(umax, u);
@@ -414,7 +416,10 @@ __device__ __forceinline__ void column_span(const ViewProj& m, const JosephView&
 // in one slice with a common minor-1 index: each candidate ray of the stack's
 // detector box is loaded once, its minor-1 weight computed once, and only the
 // minor-2 weight is evaluated per voxel.  Views whose main axis is z take
-// the voxels one at a time.
+// the voxels one at a time.  Bound: issue and the latency of the candidate loads.
+// Tilted, 181 x 167 x 149 and 120 views of 279 x 245: 3.78 ms with three columns a step (six loads in
+// flight, the walk over rows by pointer), 4.24 with one ray a step, 4.52 with one
+// ray a step by pointer.
 template <int ZV>
 __global__ void __launch_bounds__(256) joseph_bp_kernel(const float* __restrict__ vl,
     const float4* __restrict__ rays, const ViewProj* __restrict__ vp,
@@ -443,14 +448,25 @@ __global__ void __launch_bounds__(256) joseph_bp_kernel(const float* __restrict_
             float jq[ZV], accv[ZV];
 #pragma unroll
             for (int q = 0; q < ZV; ++q) { jq[q] = static_cast<float>(z0 + q); accv[q] = 0.f; }
-            for (int iv = v0; iv <= v1; ++iv) {
-                const int row = iv * nu;
-                for (int iu = u0; iu <= u1; ++iu) {
-                    const float4 r = __ldg(rk + row + iu);
-                    const float t = __ldg(vk + row + iu) * hat_weight(fmaf(r.x, c0, r.y), j1f);
-                    const float f2 = fmaf(r.z, c0, r.w);
+            // three columns at a time: two or three reach a voxel when a column is
+            // 0.7 to 1 voxel wide there
+#pragma unroll 1
+            for (int u = u0; u <= u1; u += 3) {
+                const float4* rr = rk + v0 * nu + u;
+                const float* vr = vk + v0 * nu + u;
+                const int in1 = u + 1 <= u1 ? 1 : 0, in2 = u + 2 <= u1 ? 2 : 0;
+#pragma unroll 1
+                for (int n = v1 - v0; n >= 0; --n, rr += nu, vr += nu) {
+                    const float4 ra = __ldg(rr), rb = __ldg(rr + in1), rc = __ldg(rr + in2);
+                    const float va = __ldg(vr), vb = __ldg(vr + in1), vc = __ldg(vr + in2);
+                    const float ta = va * hat_weight(fmaf(ra.x, c0, ra.y), j1f);
+                    const float tb = in1 ? vb * hat_weight(fmaf(rb.x, c0, rb.y), j1f) : 0.f;
+                    const float tc = in2 ? vc * hat_weight(fmaf(rc.x, c0, rc.y), j1f) : 0.f;
+                    const float fa = fmaf(ra.z, c0, ra.w), fb = fmaf(rb.z, c0, rb.w), fc = fmaf(rc.z, c0, rc.w);
 #pragma unroll
-                    for (int q = 0; q < ZV; ++q) accv[q] = fmaf(t, hat_weight(f2, jq[q]), accv[q]);
+                    for (int q = 0; q < ZV; ++q)
+                        accv[q] = fmaf(tc, hat_weight(fc, jq[q]), fmaf(tb, hat_weight(fb, jq[q]),
+                            fmaf(ta, hat_weight(fa, jq[q]), accv[q])));
                 }
             }
 #pragma unroll
