@@ -888,7 +888,7 @@ YKB_API size_t ykb_joseph_workspace_bytes(const ykb_joseph_plan* p)
     if (!p) return 0;
     return p->views.bytes + p->view_proj.bytes + p->rays.bytes + p->lens.bytes +
         p->weighted.bytes + p->cols.bytes + p->heights.bytes + p->vt.bytes + p->slab_x.bytes + p->slab_y.bytes +
-        p->world_views.bytes + p->siddon_vt.bytes +
+        p->world_views.bytes +
         p->fdk_coef.bytes +
         p->pseudo_coef.bytes + p->pairs.bytes + p->err_flag.bytes;
 }
@@ -1000,19 +1000,32 @@ ykb_status pseudo_bp(ykb_joseph_plan* p, const float* d_proj, float* d_volume, i
     return YKB_OK;
 }
 
-// The volume copy of the Siddon pair by detector columns; without room for it
-// the rays are walked one by one.
-ykb_status prepare_siddon_lines(ykb_joseph_plan* p, const VolumeGrid& g, cudaStream_t s)
+// The views and, for the pair by detector columns, its volume copy, in one
+// allocation; without room for the copy the rays are walked one by one.
+ykb_status prepare_siddon(ykb_joseph_plan* p, const VolumeGrid& g, cudaStream_t s)
 {
-    p->siddon_lines = 0;
-    if (!siddon_lines_apply(p->cone_views.data(), p->n_views, p->nv, g)) return YKB_OK;
-    if (p->siddon_vt.alloc(2 * sizeof(float) * joseph_line_elems(p->volume)) != cudaSuccess) {
+    const size_t views = sizeof(ykb_cone_view) * p->cone_views.size();
+    const size_t at = (views + 255) / 256 * 256;
+    const size_t copy = siddon_lines_apply(p->cone_views.data(), p->n_views, p->nv, g)
+        ? 2 * sizeof(float) * joseph_line_elems(p->volume) : 0;
+    bool lines = copy > 0;
+    cudaError_t e = cudaSuccess;
+    if (lines && !p->siddon_done) e = cudaEventCreateWithFlags(&p->siddon_done, cudaEventDisableTiming);
+    if (e != cudaSuccess) return cuda_status(e, "cudaEventCreate (Siddon)");
+    if (lines && p->world_views.alloc(at + copy) != cudaSuccess) {
         cudaGetLastError();
-        return YKB_OK;
+        lines = false;
     }
-    YKB_TRY_CUDA(cudaEventCreateWithFlags(&p->siddon_done, cudaEventDisableTiming));
-    YKB_TRY_CUDA(cudaMemsetAsync(p->siddon_vt.ptr, 0, p->siddon_vt.bytes, s));
-    p->siddon_lines = 1;
+    if (!lines && (e = p->world_views.alloc(views)) != cudaSuccess)
+        return cuda_status(e, "cudaMalloc (Siddon views)");
+    e = cudaMemcpyAsync(p->world_views.ptr, p->cone_views.data(), views, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess && lines) e = cudaMemsetAsync(p->world_views.as<char>() + at, 0, copy, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) {
+        p->world_views.reset();
+        return cuda_status(e, "cudaMemcpy (Siddon views)");
+    }
+    p->siddon_vt = lines ? reinterpret_cast<float*>(p->world_views.as<char>() + at) : nullptr;
     return YKB_OK;
 }
 
@@ -1020,26 +1033,15 @@ ykb_status siddon(ykb_joseph_plan* p, bool forward, const float* d_in, float* d_
     int accumulate, cudaStream_t s)
 {
     const std::lock_guard<std::mutex> lock(p->siddon_mutex);
-    if (!p->world_views.ptr) {
-        const size_t bytes = sizeof(ykb_cone_view) * p->cone_views.size();
-        cudaError_t e = p->world_views.alloc(bytes);
-        if (e != cudaSuccess) return cuda_status(e, "cudaMalloc (Siddon views)");
-        e = cudaMemcpyAsync(p->world_views.ptr, p->cone_views.data(), bytes, cudaMemcpyHostToDevice, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) {
-            p->world_views.reset();
-            return cuda_status(e, "cudaMemcpy (Siddon views)");
-        }
-    }
     const VolumeGrid g = make_grid(p->volume);
+    if (!p->world_views.ptr)
+        if (const ykb_status st = prepare_siddon(p, g, s)) return st;
     const ykb_cone_view* v = p->world_views.as<ykb_cone_view>();
-    if (p->siddon_lines < 0)
-        if (const ykb_status st = prepare_siddon_lines(p, g, s)) return st;
     // a graph may be replayed beside other calls of the plan, which no event
     // orders then: a captured call takes the walk, which shares no workspace
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     YKB_TRY_CUDA(cudaStreamIsCapturing(s, &capture));
-    if (p->siddon_lines == 0 || capture != cudaStreamCaptureStatusNone) {
+    if (!p->siddon_vt || capture != cudaStreamCaptureStatusNone) {
         if (forward)
             YKB_TRY_CUDA(launch_siddon_fp(d_in, v, p->n_views, p->nu, p->nv, g, d_out, accumulate, s));
         else
@@ -1047,7 +1049,7 @@ ykb_status siddon(ykb_joseph_plan* p, bool forward, const float* d_in, float* d_
         return YKB_OK;
     }
     YKB_TRY_CUDA(cudaStreamWaitEvent(s, p->siddon_done, 0));
-    float* vt = p->siddon_vt.as<float>();
+    float* const vt = p->siddon_vt;
     if (forward)
         YKB_TRY_CUDA(launch_siddon_fp_lines(d_in, vt, v, p->n_views, p->nu, p->nv, g, d_out, accumulate, s));
     else

@@ -230,7 +230,7 @@ cudaError_t fdk_tma_box(const FdkViewCoef* coef, int n_views, const VolumeGrid& 
 size_t fdk_tma_part_floats(const VolumeGrid& g, int n_views);
 // Limit of the TMA backprojection's pipeline waits (a wait that runs out
 // sets the error word and stops the CTA) and, for tests of that path, a view
-// whose copy the producer withholds (-1: none).  Waits that drain copies in
+// whose copy is withheld (-1: none).  Waits that drain copies in
 // flight keep the default limit.
 struct PipelineWait {
     unsigned long long limit_ns = 2000000000ull;
@@ -444,11 +444,10 @@ struct ykb_joseph_plan {
     ykb::DeviceBuffer slab_y, slab_x;  // transposed volume copies (scans without fp_lines)
     ykb::JosephFpLines fp_lines;       // forward projection by lines (column_bp scans)
     ykb::DeviceBuffer vt;              // its volume copy [x][y][z]
-    // Siddon, set up on first use: the views, and for axial-column scans a volume
-    // copy.  Calls on different streams take turns on the copy
-    ykb::DeviceBuffer world_views;     // ykb_cone_view[n]
-    int siddon_lines = -1;             // by detector columns: 1, ray by ray: 0, undecided: -1
-    ykb::DeviceBuffer siddon_vt;
+    // Siddon, set up on first use: the views, and for untilted scans a volume copy
+    // behind them.  Calls on different streams take turns on the copy
+    ykb::DeviceBuffer world_views;     // ykb_cone_view[n], then the copy
+    float* siddon_vt = nullptr;        // (null: the rays are walked one by one)
     cudaEvent_t siddon_done = nullptr; // the last call's work on the copy
     std::mutex siddon_mutex;
     ~ykb_joseph_plan() { if (siddon_done) cudaEventDestroy(siddon_done); }
