@@ -606,20 +606,21 @@ def main():
     bp_bytes = 4.0 * w.n_views * w.n_det ** 2 + 4.0 * w.n_vox ** 3
     achieved = bp_bytes / (bp_step_ms * 1e-3) / 1e9
     # DRAM traffic of one launch: ncu (dram__bytes_read + write) on the
-    # 256^3 x 360 x 384^2 case gave 703.4 + 64.8 MB against 279.4 MB
-    # compulsory (tap-pair rows are 8 B per sample; L2 misses re-read some
-    # rows); scaled by the compulsory bytes of one launch, which grow in
-    # proportion
-    traffic = 768.2e6 * (bp_bytes / stages["groups_per_step"]) / (
+    # 256^3 x 360 x 384^2 case gave 653.6 MB read and 127.6 MB written, of
+    # which 60.5 MB are sums of split views that larger volumes do not write,
+    # against 279.4 MB compulsory (row pairs are 8 B per sample; L2 misses
+    # re-read some rows); scaled by the compulsory bytes of one launch, which
+    # grow in proportion
+    traffic = 720.7e6 * (bp_bytes / stages["groups_per_step"]) / (
         4.0 * 360 * 384 * 384 + 4.0 * 256 ** 3)
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / peaks["hbm_gbs"], "traffic": traffic, "peak_source": peak_src,
                 "traffic_source": "ncu 256^3x360x384^2 capture scaled by compulsory bytes",
-                "kernel": "fdk_bp_tma_kernel (TMA-staged tap pairs)", "kernel_ms": ms_bp,
+                "kernel": "fdk_bp_tma_kernel (TMA-staged row pairs)", "kernel_ms": ms_bp,
                 "kernel_ms_source": "CUDA events around its launch inside the FDK steps",
                 "algorithmic_bytes_per_launch": bp_bytes / stages["groups_per_step"]}
     # the bound that binds: 16 B of bilinear taps per update, loaded from
-    # shared memory as two 8-byte tap pairs, against the measured 8-byte
+    # shared memory as two 8-byte row pairs, against the measured 8-byte
     # shared-load bandwidth of this GPU
     import ctypes as C
     smem = C.c_double(0.0)
@@ -683,7 +684,7 @@ def main():
 
 def plan_chunk_views(w) -> int:
     """Views per workspace chunk of an FDK plan: a budget of 8 GiB at 12 bytes
-    per detector pixel (preweighted rows + filtered tap pairs)."""
+    per detector pixel (preweighted rows + filtered row pairs)."""
     return max(1, min(w.n_views, (8 << 30) // (12 * w.n_det * w.n_det)))
 
 

@@ -1,6 +1,6 @@
 // Shared-memory load bandwidth of this GPU, measured: the on-chip peak that
-// the FDK backprojection (two 8-byte shared loads of bilinear tap pairs per
-// voxel update) is reported against.
+// the FDK backprojection (two 8-byte shared loads of row pairs per voxel
+// update) is reported against.
 //
 // Every CTA fills 16 KB of shared memory and its 256 threads stream it back
 // with vector loads: lane i reads the WORDS 32-bit words at word offset

@@ -242,7 +242,7 @@ YKB_API ykb_status ykb_fdk_stage_times(ykb_fdk_plan* plan, ykb_stream stream,
 
 /* Test hook for the timeout path of the TMA backprojection: sets the limit
  * of its pipeline waits to wait_ns (0 restores the default, about 2 s) and,
- * when withheld_view >= 0, makes the copy producer skip that view (an index
+ * when withheld_view >= 0, withholds the copy of that view (an index
  * within each backprojection launch) so that every wait for it runs out.  A
  * wait that runs out sets the plan's error word, which ykb_fdk_check
  * reports; the kernel ends without hanging, its copies in flight drained, and
@@ -324,8 +324,8 @@ typedef enum ykb_task {
  *     area (fdk_pseudo_matched_bp_launch, src/FlatFpBp/BP/kernels/
  *     YkBpFdkKernel.cu:356-450,532-548), an approximate transpose of the
  *     forward projector.  Its first call builds the plan's tables for it
- *     (synchronising the stream) and a tap-pair copy of the projections
- *     (8 bytes per pixel).
+ *     (synchronising the stream) and room for a row-pair copy of the
+ *     projections (8 bytes per pixel).
  * Other task values return YKB_ERR_UNSUPPORTED. */
 YKB_API ykb_status ykb_operator_apply(ykb_joseph_plan* plan, int task,
     const float* d_in, float* d_out, int accumulate, ykb_stream stream);
@@ -371,7 +371,7 @@ YKB_API ykb_status ykb_cgls_update_p(ykb_iter* ctx, const double* d_gamma_new,
  * SMs): 4 CTAs per SM stream 16 KB of shared memory with conflict-free
  * vector loads of bytes_per_lane (8 or 16) bytes, best of five timed
  * launches (CUDA events) after one warm-up.  The on-chip peak that the
- * backprojection's two 8-byte tap-pair loads per voxel update are reported
+ * backprojection's two 8-byte row-pair loads per voxel update are reported
  * against.  Synchronous; no counterpart in the reference. */
 YKB_API ykb_status ykb_measure_shared_load_gbs(int device, int bytes_per_lane, double* gbs);
 
