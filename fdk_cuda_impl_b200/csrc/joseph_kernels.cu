@@ -791,11 +791,12 @@ __global__ void __launch_bounds__(kLineThreads, 3) joseph_bp_lines_kernel(
 //   * the last warp, which the lines rarely reach, prepares the next view's
 //     boxes, and every thread has its next line's first rays in flight while it
 //     sums its column: two barriers a view.
-// Bound: instruction issue and the shared-memory data path together (55 and 66 %;
+// Bound: instruction issue and the shared-memory data path together (59 and 62 %;
 // three wavefronts a request in the column sums), with 24 warps an SM.  256^3 x
-// 360 x 384^2: 21.1 ms, before 24.9; the runs alone, without the last two points:
-// 25.2; (a2, e2) from the 16-byte ray records instead of a table of their own: 22.2;
-// two sets of rays in turn instead of a copy of the set in flight: 22.1 (spills).
+// 360 x 384^2: 20.2 ms, before 24.9; scalar instead of packed sums of the two
+// slices: 20.5; the runs alone, without the last two points: 25.2; (a2, e2) from
+// the 16-byte ray records instead of a table of their own: 22.2 against 21.1; two
+// sets of rays in turn instead of a copy of the set in flight: 22.1 (spills).
 // ---------------------------------------------------------------------------
 constexpr int kRunGroup = 4;  // rays of a line loaded together
 
@@ -947,15 +948,13 @@ struct RunSums {
             const f2 f = f2pack(fmaf(r.a[q].x, csa, r.a[q].y), fmaf(r.a[q].x, csb, r.a[q].y));
             const f2 t = f2add_rm(f, M);
             const f2 vv = f2pack(r.v[q], r.v[q]), u = f2mul(vv, f2sub(f, f2sub(t, M)));
-            float tt[2], uu[2], xx[2];
+            float tt[2];
             f2unpack(t, tt[0], tt[1]);
-            f2unpack(u, uu[0], uu[1]);
-            f2unpack(f2sub(vv, u), xx[0], xx[1]);
+            const bool ba = tt[0] != cur[0], bb = tt[1] != cur[1];  // the next voxel begins
+            f2unpack(f2add(f2pack(ba ? hi[0] : lo[0], bb ? hi[1] : lo[1]), f2sub(vv, u)), lo[0], lo[1]);
+            f2unpack(f2add(f2pack(ba ? 0.f : hi[0], bb ? 0.f : hi[1]), u), hi[0], hi[1]);
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                const bool begins = tt[e] != cur[e];  // the next voxel
-                lo[e] = (begins ? hi[e] : lo[e]) + xx[e];
-                hi[e] = (begins ? 0.f : hi[e]) + uu[e];
                 cur[e] = tt[e];
                 // slot ZC + 1 takes what falls outside
                 const uint32_t slot = min(__float_as_uint(tt[e]) - slot0, static_cast<uint32_t>(ZC + 1));
