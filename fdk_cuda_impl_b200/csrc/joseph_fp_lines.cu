@@ -118,7 +118,7 @@ __device__ __forceinline__ void sample_slices(const f2 (&a2)[kCols / 2], const f
 __device__ __noinline__ float line_entry(const float* __restrict__ vt, long st_1, int nz, int2 t, int z)
 {
     if (z < 0 || z >= nz) return 0.f;
-    const float* p = vt + 4 * static_cast<long>(t.x) + z;
+    const float* p = vt + 4 * static_cast<long>(static_cast<uint32_t>(t.x)) + z;
     return fmaf(__int_as_float(t.y), p[st_1] - p[0], p[0]);
 }
 __device__ __forceinline__ void sample_volume(const float* __restrict__ vt, long st_1, int nz,
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(kMaxRows, 2) joseph_fp_lines_kernel(const floa
         const bool in = s <= last && f1 > -1.f && f1 < static_cast<float>(n1);
         const long row = (s + kLinePad) * st_s + (static_cast<int>(fl) + kLinePad) * st_1;
         tables[(b % kTables) * 32 + lane] =
-            in ? make_int2(static_cast<int>(row / 4), __float_as_int(f1 - fl)) : make_int2(0, 0);
+            in ? make_int2(static_cast<int>(joseph_line_quad(row)), __float_as_int(f1 - fl)) : make_int2(0, 0);
     };
     if (warp == 0) {
         form_table(0);
@@ -264,10 +264,10 @@ __global__ void __launch_bounds__(kMaxRows, 2) joseph_fp_lines_kernel(const floa
                 if (z >= 0 && z < nz) {  // else above or below the volume (its rows are padded to quads)
                     const float4* const src = reinterpret_cast<const float4*>(vt + z);
                     const float4* const src1 = reinterpret_cast<const float4*>(vt + z + st_1);
-                    p0 = __ldg(src + t.x);
-                    r0 = __ldg(src1 + t.x);
-                    p1 = __ldg(src + t.z);
-                    r1 = __ldg(src1 + t.z);
+                    p0 = __ldg(src + static_cast<uint32_t>(t.x));
+                    r0 = __ldg(src1 + static_cast<uint32_t>(t.x));
+                    p1 = __ldg(src + static_cast<uint32_t>(t.z));
+                    r1 = __ldg(src1 + static_cast<uint32_t>(t.z));
                 }
                 const float w0 = __int_as_float(t.y), w1 = __int_as_float(t.w);
                 *reinterpret_cast<float4*>(out) = make_float4(fmaf(w0, r0.x - p0.x, p0.x),

@@ -830,7 +830,7 @@ YKB_API ykb_status ykb_joseph_plan_create(const ykb_cone_view* views, int n_view
         p->column_bp = e == cudaSuccess && differs == 0;
         if (!p->column_bp) p->cols.reset();
         if (p->column_bp) {
-            p->fp_lines = joseph_fp_lines_shape(p->host_views, nv);
+            if (joseph_line_volume_fits(*volume)) p->fp_lines = joseph_fp_lines_shape(p->host_views, nv);
             // (32-bit byte offsets of a view's ray records)
             p->bp_runs = static_cast<long>(nu) * nv < (1L << 27) && joseph_bp_runs(p->host_views, nv);
             // without room for the table the ray records serve

@@ -300,6 +300,14 @@ inline size_t joseph_line_elems(const ykb_volume& v)
 {
     return static_cast<size_t>(v.nx + 2 * kLinePad) * (v.ny + 2 * kLinePad) * joseph_line_pitch(v.nz);
 }
+// The lines' tables name a row of the copy by its first quad, in 32 unsigned bits
+constexpr uint32_t joseph_line_quad(long row) { return static_cast<uint32_t>(row / 4); }
+// Volumes whose copy they reach, and whose y fits the third dimension of the copy's
+// launch; the slab kernel projects the others
+inline bool joseph_line_volume_fits(const ykb_volume& v)
+{
+    return v.ny <= 65535 && joseph_line_elems(v) <= (size_t(1) << 34);
+}
 cudaError_t launch_joseph_line_volume(const float* vol, int nx, int ny, int nz, float* vt, cudaStream_t s);
 // vt: joseph_line_elems floats, zeroed once; every call rewrites its interior
 cudaError_t launch_joseph_fp_lines(const float* vol, int nx, int ny, int nz, float* vt,

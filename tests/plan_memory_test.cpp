@@ -1,0 +1,145 @@
+// The plans' choices of buffers and kernels, without a GPU: ykb_api.cpp and
+// ykb_geometry.cpp linked with a fake CUDA runtime, whose device memory is a
+// number of bytes, and fake launchers, which count their calls.
+#include <algorithm>
+#include <cstdio>
+#include <cstring>
+#include <map>
+
+#include "ykb_internal.hpp"
+
+namespace {
+
+size_t g_capacity = ~size_t(0), g_used = 0;
+std::map<void*, size_t> g_blocks;
+int g_failures = 0;
+
+void expect(bool ok, const char* what)
+{
+    if (!ok) {
+        ++g_failures;
+        std::fprintf(stderr, "FAILED: %s\n", what);
+    }
+}
+
+} // namespace
+
+extern "C" {
+cudaError_t cudaGetDeviceCount(int* n) { *n = 1; return cudaSuccess; }
+cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+const char* cudaGetErrorName(cudaError_t) { return "error"; }
+const char* cudaGetErrorString(cudaError_t) { return "error"; }
+cudaError_t cudaMalloc(void** p, size_t n)
+{
+    if (g_used + n > g_capacity) return cudaErrorMemoryAllocation;
+    static char* next = reinterpret_cast<char*>(size_t(1) << 40);
+    *p = next;
+    next += (n + 511) / 512 * 512;
+    g_blocks[*p] = n;
+    g_used += n;
+    return cudaSuccess;
+}
+cudaError_t cudaFree(void* p)
+{
+    g_used -= g_blocks.at(p);
+    g_blocks.erase(p);
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpy(void*, const void*, size_t, cudaMemcpyKind) { return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void* to, const void*, size_t n, cudaMemcpyKind kind, cudaStream_t)
+{
+    if (kind == cudaMemcpyDeviceToHost) std::memset(to, 0, n);
+    return cudaSuccess;
+}
+cudaError_t cudaMemset(void*, int, size_t) { return cudaSuccess; }
+cudaError_t cudaMemsetAsync(void*, int, size_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = nullptr; return cudaSuccess; }
+cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+}
+
+namespace ykb {
+cudaError_t launch_joseph_ray_table(const JosephView*, int, int, int, float4*, float*, cudaStream_t)
+{
+    return cudaSuccess;
+}
+cudaError_t launch_joseph_column_table(const float4*, int, int, int, float2*, int*, cudaStream_t)
+{
+    return cudaSuccess;
+}
+cudaError_t launch_joseph_ray_heights(const float4*, long, float2*, cudaStream_t) { return cudaSuccess; }
+JosephFpLines joseph_fp_lines_shape(const std::vector<JosephView>&, int) { return {128, 144}; }
+bool joseph_bp_runs(const std::vector<JosephView>&, int) { return true; }
+int joseph_bp_splits(const ykb_volume&, int) { return 4; }
+} // namespace ykb
+
+using namespace ykb;
+
+namespace {
+
+struct Scan {
+    std::vector<ykb_cone_view> views;
+    int nu, nv;
+    ykb_volume volume{};
+    Scan(int n_views, int nu_, int nv_, int nx, int ny, int nz) : views(n_views), nu(nu_), nv(nv_)
+    {
+        ykb_circular_flat spec{};
+        spec.total_views = spec.views_per_turn = n_views;
+        spec.rotation_direction = 1;
+        spec.sid_mm = 500.f;
+        spec.sdd_mm = 1000.f;
+        spec.channels = nu;
+        spec.rows = nv;
+        spec.channel_size_mm = spec.row_size_mm = 0.1f;
+        expect(ykb_build_circular_flat(&spec, views.data(), n_views) == YKB_OK, "views");
+        volume.nx = nx; volume.ny = ny; volume.nz = nz;
+        volume.vox_x = volume.vox_y = volume.vox_z = 100.f / std::max({nx, ny, nz});
+    }
+    ykb_joseph_plan* joseph(size_t capacity = ~size_t(0)) const
+    {
+        g_capacity = capacity;
+        ykb_joseph_plan* p = nullptr;
+        const ykb_status st = ykb_joseph_plan_create(views.data(), static_cast<int>(views.size()), nu, nv,
+            &volume, 0, &p);
+        expect((st == YKB_OK) == (p != nullptr), "a plan or an error");
+        return p;
+    }
+};
+
+// The line projector's copy where 32 unsigned bits of quads reach all of it, the
+// slabs where they do not
+void line_volume()
+{
+    for (int n : {64, 2048, 2500, 2700}) {
+        const Scan scan(4, 32, 32, n, n, n);
+        ykb_joseph_plan* p = scan.joseph();
+        if (!p) continue;
+        const bool fits = n <= 2500;
+        expect((p->vt.ptr != nullptr) == fits && (p->fp_lines.rows > 0) == fits, "line copy or not");
+        expect((p->slab_x.ptr != nullptr && p->slab_y.ptr != nullptr) == !fits, "slabs or not");
+        if (fits) {
+            // the first element of the copy's last row
+            const long row = static_cast<long>(joseph_line_elems(scan.volume)) - joseph_line_pitch(n);
+            expect(4 * static_cast<long>(joseph_line_quad(row)) == row, "quad of the last row");
+        }
+        ykb_joseph_plan_destroy(p);
+    }
+    const Scan tall(4, 32, 32, 8, 70000, 8);
+    if (ykb_joseph_plan* p = tall.joseph()) {
+        expect(p->fp_lines.rows == 0, "y past the launch's third dimension");
+        ykb_joseph_plan_destroy(p);
+    }
+    expect(g_used == 0 && g_blocks.empty(), "everything given back");
+}
+
+} // namespace
+
+int main(int argc, char** argv)
+{
+    const std::string what = argc > 1 ? argv[1] : "";
+    if (what == "line_volume") line_volume();
+    else return 2;
+    return g_failures ? 1 : 0;
+}
