@@ -218,7 +218,7 @@ bool small_volume(const VolumeGrid& g)
 // crossings of flat rays keep their place.
 // Bound: instruction issue (22 a segment and ray, 63 % in the projector, 71 % in
 // the backprojector, whose reductions keep L2 half busy).  256^3 x 120 x 384^2:
-// 5.3 and 6.5 ms, before 7.3 and 11.9; error against FP64 7.5e-7, before 7.7e-7
+// 5.2 and 6.7 ms, before 7.3 and 11.9; error against FP64 7.5e-7, before 7.7e-7
 // (8.1e-7 while the face distances were rounded once per axis).
 // ---------------------------------------------------------------------------
 constexpr int kLineCols = 4;
@@ -272,7 +272,8 @@ __device__ __forceinline__ void column_start(const ykb_cone_view& v, int iu, con
     w.stepY = sy * nzp;
 }
 
-// the next segment: its end and its row; past the exit, empty ones
+// the next segment: its end and its row; past the exit, empty ones in the zero row
+// at the copy's start
 __device__ __forceinline__ float2 column_segment(ColumnWalk& w)
 {
     const float2 out = make_float2(fmaxf(w.s, fminf(fminf(w.sX, w.sY), w.smax)), __int_as_float(w.row));
@@ -286,6 +287,8 @@ __device__ __forceinline__ float2 column_segment(ColumnWalk& w)
             w.jy += 1.f;
             w.sY = w.jy < w.mY ? fmaf(w.jy, w.dY, fmaf(w.jy, w.loY, w.aY)) : 3e38f;
         }
+    } else {
+        w.row = 0;
     }
     w.s = out.x;
     return out;
@@ -327,19 +330,29 @@ __device__ __forceinline__ void line_ray(const ykb_cone_view& v, int iu, int iv,
 }
 
 // One segment of a ray: the voxel it enters in (i0, weight w0) and the one it
-// leaves in (i1, w1; crosses is false when they are the same and w1 is zero).
-// Indices are z.
-struct LineStep { int i0, i1; float w0, w1; bool crosses; };
+// leaves in (i1, w1), indices in z.  Where they are the same, the projector has
+// the whole length in w0 (in1 false: one gather); the backprojector has it in
+// either, from the same expression held between zero and the segment's length: no
+// weight is negative where the face rounds to a place outside the segment, and
+// one that is zero marks a voxel that is not crossed.
+struct LineStep { int i0, i1; float w0, w1; bool in1; };
+template <bool FORWARD>
 __device__ __forceinline__ LineStep line_step(LineRay& r, float s1)
 {
     LineStep st;
     const float t1 = __fadd_rd(fmaf(s1, r.mz, r.ze), kFloorMagic);
     st.i0 = __float_as_int(r.t) - kFloorMagicBits + r.zref;
     st.i1 = __float_as_int(t1) - kFloorMagicBits + r.zref;
-    st.crosses = t1 != r.t;
-    const float face = fmaxf(t1, r.t) - kFloorMagic;
-    st.w1 = st.crosses ? s1 - (face - r.ze) * r.inv : 0.f;
-    st.w0 = (s1 - r.s) - st.w1;
+    const float face = fmaxf(t1, r.t) - kFloorMagic, length = s1 - r.s;
+    st.w1 = s1 - (face - r.ze) * r.inv;
+    if constexpr (FORWARD) {
+        st.in1 = t1 != r.t;
+        if (!st.in1) st.w1 = 0.f;
+    } else {
+        st.w1 = fminf(fmaxf(st.w1, 0.f), length);
+        st.in1 = st.w1 != 0.f;
+    }
+    st.w0 = length - st.w1;
     r.s = s1;
     r.t = t1;
     return st;
@@ -395,17 +408,17 @@ __global__ void __launch_bounds__(kLineRows + 32, 6) siddon_lines_kernel(const f
 #pragma unroll
                 for (int c = 0; c < kLineCols; ++c) {
                     const float2 e = seg[q][c];
-                    const LineStep st = line_step(r[c], e.x);
+                    const LineStep st = line_step<FORWARD>(r[c], e.x);
                     const int row = __float_as_int(e.y);
                     const bool in0 = !decltype(checked)::value ||
                         static_cast<unsigned>(st.i0) < static_cast<unsigned>(g.nz);
-                    const bool in1 = st.crosses && (!decltype(checked)::value ||
+                    const bool in1 = st.in1 && (!decltype(checked)::value ||
                         static_cast<unsigned>(st.i1) < static_cast<unsigned>(g.nz));
                     if constexpr (FORWARD) {
                         if (in0) acc[c] = fmaf(__ldg(in + (row + st.i0)), st.w0, acc[c]);
                         if (in1) acc[c] = fmaf(__ldg(in + (row + st.i1)), st.w1, acc[c]);
                     } else {
-                        if (in0 && p[c] != 0.f) atomicAdd(out + (row + st.i0), p[c] * st.w0);
+                        if (in0 && st.w0 != 0.f && p[c] != 0.f) atomicAdd(out + (row + st.i0), p[c] * st.w0);
                         if (in1 && p[c] != 0.f) atomicAdd(out + (row + st.i1), p[c] * st.w1);
                     }
                 }

@@ -70,3 +70,32 @@ def test_siddon_pair_matches_oracle(oracle, cuda_device, case):
         hit = plan.forward_siddon((xd * 0 + 1) * (~torch.isfinite(bad)))
         assert torch.isfinite(plan.forward_siddon(bad)[hit == 0]).all()
     plan.close()
+
+
+@pytest.mark.parametrize("n", [21, 48, 75])
+def test_infinite_values_stay_where_rays_cross(cuda_device, n):
+    # infinite pixels make infinite exactly the voxels that their rays cross,
+    # infinite voxels the pixels whose rays cross them; no NaN (infinity times a
+    # length of zero), no -inf (a length below zero)
+    import torch
+    from fdk_cuda_impl_b200.projectors import JosephPlan
+    scan = CircularScan(9, 9, 500.0, 1000.0, n + 5, n, 300.0 / n, 280.0 / n, start_angle_rad=0.03)
+    grid = VolumeGrid(n, n + 3, n - 7, (128.0 / n,) * 3, (0.4, -0.7, 0.2))
+    plan = JosephPlan(scan.views(), n + 5, n, grid)
+
+    def check(apply, data):
+        one = apply(data)
+        inf = apply(torch.where(data > 0, torch.inf, 0.0))
+        assert float(one.min()) >= 0 and float(one.max()) > 0
+        assert not torch.isnan(inf).any() and float(inf.min()) >= 0
+        assert torch.equal(one != 0, torch.isinf(inf))
+
+    for k in range(9):
+        y = torch.zeros(plan.proj_shape, device="cuda")
+        y[k] = 1.0
+        check(plan.backproject_siddon, y)
+    for at in [(n // 2 - 3, n // 2, n // 2), (n // 3, n // 4, n // 2), (n // 2, n // 2, n // 5)]:
+        x = torch.zeros(grid.shape, device="cuda")
+        x[tuple(slice(i - 1, i + 2) for i in at)] = 1.0
+        check(plan.forward_siddon, x)
+    plan.close()
