@@ -192,12 +192,6 @@ __device__ __forceinline__ f2 f2add_rm(f2 a, f2 b)
     asm("add.rm.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
-__device__ __forceinline__ f2 f2mul(f2 a, f2 b)
-{
-    f2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
 
 // 1.5 * 2^23: for |x| < 2^22, x + kMagic holds round(x) in its low mantissa
 // bits; (f - 1/2) + kMagic thus holds floor(f), except at integer f where
@@ -942,17 +936,19 @@ struct RunSums {
     __device__ __forceinline__ void add(const RunRays& r, float csa, float csb, uint32_t slot0, float* La,
         float* Lb)
     {
-        const f2 M = f2pack(kMagic, kMagic);
+        const f2 M = f2pack(kMagic, kMagic), one = f2pack(1.f, 1.f);
 #pragma unroll
         for (int q = 0; q < kRunGroup; ++q) {
             const f2 f = f2pack(fmaf(r.a[q].x, csa, r.a[q].y), fmaf(r.a[q].x, csb, r.a[q].y));
             const f2 t = f2add_rm(f, M);
-            const f2 vv = f2pack(r.v[q], r.v[q]), u = f2mul(vv, f2sub(f, f2sub(t, M)));
+            // v (1 - w) and v w, each a product of its own: an infinite v stays
+            // infinite where v - v w would be NaN
+            const f2 vv = f2pack(r.v[q], r.v[q]), w = f2sub(f, f2sub(t, M));
             float tt[2];
             f2unpack(t, tt[0], tt[1]);
             const bool ba = tt[0] != cur[0], bb = tt[1] != cur[1];  // the next voxel begins
-            f2unpack(f2add(f2pack(ba ? hi[0] : lo[0], bb ? hi[1] : lo[1]), f2sub(vv, u)), lo[0], lo[1]);
-            f2unpack(f2add(f2pack(ba ? 0.f : hi[0], bb ? 0.f : hi[1]), u), hi[0], hi[1]);
+            f2unpack(f2fma(vv, f2sub(one, w), f2pack(ba ? hi[0] : lo[0], bb ? hi[1] : lo[1])), lo[0], lo[1]);
+            f2unpack(f2fma(vv, w, f2pack(ba ? 0.f : hi[0], bb ? 0.f : hi[1])), hi[0], hi[1]);
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 cur[e] = tt[e];

@@ -85,3 +85,24 @@ def test_line_backprojector_matches_gather(oracle, cuda_device, monkeypatch, cas
     assert torch.equal(lines.adjoint(torch.zeros_like(y)), torch.zeros_like(b))
     lines.close()
     gather.close()
+
+
+@pytest.mark.parametrize("runs", [True, False])
+def test_infinite_rays_stay_infinite(cuda_device, runs):
+    # A^T of infinite rays: infinite exactly where their weights are not zero, no
+    # NaN (v - v w of an infinite v), with rows closer than a voxel (lines formed
+    # in runs) and farther apart.  Rays through voxel centres have a weight of
+    # zero times infinity: the offsets keep them off
+    import torch
+    from fdk_cuda_impl_b200.projectors import JosephPlan
+    pix = 0.9 if runs else 3.1
+    scan = CircularScan(8, 8, 500.0, 1000.0, 40, 36, 1.7, pix, start_angle_rad=0.05)
+    grid = VolumeGrid(33, 30, 28, (1.0, 1.0, 1.0), (0.4, -0.7, 0.23))
+    plan = JosephPlan(scan.views(), 40, 36, grid)
+    for k in range(8):
+        y = torch.zeros(plan.proj_shape, device="cuda")
+        y[k, 3:33:3, 2:38:5] = 1.0
+        one, inf = plan.adjoint(y), plan.adjoint(torch.where(y > 0, torch.inf, 0.0))
+        assert not torch.isnan(inf).any()
+        assert torch.equal(one != 0, torch.isinf(inf))
+    plan.close()
