@@ -833,12 +833,6 @@ YKB_API ykb_status ykb_joseph_plan_create(const ykb_cone_view* views, int n_view
             if (joseph_line_volume_fits(*volume)) p->fp_lines = joseph_fp_lines_shape(p->host_views, nv);
             // (32-bit byte offsets of a view's ray records)
             p->bp_runs = static_cast<long>(nu) * nv < (1L << 27) && joseph_bp_runs(p->host_views, nv);
-            // without room for the table the ray records serve
-            if (p->heights.alloc(sizeof(float2) * rays) == cudaSuccess)
-                e = launch_joseph_ray_heights(p->rays.as<float4>(), static_cast<long>(rays),
-                    p->heights.as<float2>(), s);
-            else
-                cudaGetLastError();
         }
     }
     // the forward projector's volume copies, their zero borders written once (the
@@ -864,6 +858,17 @@ YKB_API ykb_status ykb_joseph_plan_create(const ykb_cone_view* views, int n_view
         }
         if (p->bp_splits > 1) p->bp_parts = reinterpret_cast<double*>(p->weighted.as<char>() + weighted);
         else e = p->weighted.alloc(weighted);
+    }
+    // last, when all that the plan cannot do without has its room: without a table
+    // of their own the rays' heights are read from the ray records
+    if (e == cudaSuccess && p->column_bp) {
+        if (p->heights.alloc(sizeof(float2) * rays) == cudaSuccess) {
+            e = launch_joseph_ray_heights(p->rays.as<float4>(), static_cast<long>(rays),
+                p->heights.as<float2>(), s);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        } else {
+            cudaGetLastError();
+        }
     }
     cudaStreamDestroy(s);
     if (e != cudaSuccess) {

@@ -134,12 +134,43 @@ void line_volume()
     expect(g_used == 0 && g_blocks.empty(), "everything given back");
 }
 
+// A plan is refused only when what it cannot do without has no room; the split
+// views' sums and the table of ray heights give way first
+void optional_buffers()
+{
+    const Scan scan(24, 40, 36, 64, 60, 48);
+    ykb_joseph_plan* p = scan.joseph();
+    if (!p) return;
+    expect(p->heights.ptr && p->bp_splits > 1 && p->bp_parts && p->fp_lines.rows > 0, "all with room");
+    const size_t full = g_used, heights = p->heights.bytes;
+    const size_t sums = sizeof(double) * p->bp_splits * 64 * 60 * 48;
+    ykb_joseph_plan_destroy(p);
+    for (const size_t capacity : {full, full - 1, full - heights, full - heights - 1, full - heights - sums}) {
+        p = scan.joseph(capacity);
+        expect(p != nullptr, "a plan");
+        if (!p) continue;
+        expect(g_used <= capacity && p->weighted.ptr && p->vt.ptr, "what it needs");
+        expect((p->heights.ptr != nullptr) == (capacity == full ||
+                   (capacity < full - heights && heights <= sums && capacity >= full - sums)), "heights");
+        expect((p->bp_splits > 1) == (capacity >= full - heights) &&
+                   (p->bp_parts != nullptr) == (p->bp_splits > 1), "sums");
+        expect(p->ray_heights().bytes == (p->heights.ptr ? 8 : 16), "heights read from");
+        ykb_joseph_plan_destroy(p);
+    }
+    g_capacity = full - heights - sums - 1;
+    p = nullptr;
+    expect(ykb_joseph_plan_create(scan.views.data(), 24, scan.nu, scan.nv, &scan.volume, 0, &p) ==
+               YKB_ERR_OUT_OF_MEMORY && !p, "refused below");
+    expect(g_used == 0 && g_blocks.empty(), "everything given back");
+}
+
 } // namespace
 
 int main(int argc, char** argv)
 {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "line_volume") line_volume();
+    else if (what == "optional_buffers") optional_buffers();
     else return 2;
     return g_failures ? 1 : 0;
 }
