@@ -74,3 +74,32 @@ def test_split_views_match_one_job_a_tile(oracle, cuda_device, monkeypatch, n, n
     assert K.rel_rmse(shifted.cpu().numpy(), 2.0 * b.cpu().numpy()) <= 2e-5
     split.close()
     one.close()
+
+
+@pytest.mark.parametrize("views,nu,nv,n,nz", [(8, 64, 48, 40, 32), (16, 96, 64, 64, 48)])
+def test_column_terms_round_once(oracle, cuda_device, monkeypatch, views, nu, nv, n, nz):
+    # plain rows and the pseudo-matched weight: u and v of a column are rounded to
+    # FP32 once, below 64 px (rms 2^-18 / sqrt(12) = 1.1e-6 px each).  Uniform rows
+    # in 0.5 .. 1.5 differ by 0.41 rms from pixel to pixel: 1.1e-6 x 0.41 x sqrt(2)
+    # of a view's value, averaged over the views, beside the FP32 sum's
+    # 2^-24 sqrt(views) / 3.  Several roundings a coordinate exceed it
+    import torch
+    from fdk_cuda_impl_b200.projectors import FdkPlan, JosephPlan
+    bound = ((1.1e-6 * 0.41 * 2 ** 0.5) ** 2 / views + (2.0 ** -24 / 3) ** 2 * views) ** 0.5
+    scan = CircularScan(views, views, 500.0, 1000.0, nu, nv, 300.0 / nu, 300.0 / nu,
+                        start_angle_rad=0.1, offset_unv_mm=(0.8, 0.0, -1.1))
+    grid = VolumeGrid(n, n + 3, nz, (128.0 / n,) * 3, (0.3, -0.2, 0.1))
+    table, vol = scan.views(), K.oracle_volume(oracle, grid)
+    p = oracle.uniform((views, nv, nu), 0.5, 1.5, 4)
+    pd = torch.from_numpy(p).cuda()
+    jp = JosephPlan(table, nu, nv, grid)
+    pseudo = jp.backproject_pseudo(pd).cpu().numpy()
+    jp.check()
+    jp.close()
+    assert K.rel_rmse(pseudo, oracle.pseudo_bp(table, nu, nv, vol, p)) <= bound
+    monkeypatch.setenv("YKB_FDK_BP_PATH", "rows")
+    plan = FdkPlan(table, nu, nv, scan.scan_range, grid, RampFilter())
+    rows = plan.backproject(pd).cpu().numpy()
+    plan.check()
+    plan.close()
+    assert K.rel_rmse(rows, oracle.fdk_backproject(table, nu, nv, scan.scan_range, vol, p)) <= bound
