@@ -623,7 +623,7 @@ constexpr int kSms = 148;
 // pad to 512 and 448; 96 columns of few rows as two of 64, side by side.
 // 241 views of 391 x 333 in three calls: 0.61 ms before (tiles of 64), 0.22 now;
 // 60 of 96 x 64: 13.2 and 10.9 us.
-int tile_n(int nu, long rows)
+int soonest_tile(int nu, long rows)
 {
     int best = 0;
     double best_cost = 0.0;
@@ -637,12 +637,17 @@ int tile_n(int nu, long rows)
 
 } // namespace
 
-int tc_filter_sub_batches(int nu, long rows)
+int tc_filter_tile(int nu, long rows)
+{
+    const int tn = soonest_tile(nu, rows);
+    return soonest_tile(nu, rows / tc_filter_sub_batches(tn, nu, rows));
+}
+
+int tc_filter_sub_batches(int tn, int nu, long rows)
 {
     // overlapping the preweight pays while each sub-batch still fills the GPU
     // with two rounds of tiles (180 views of 192 x 128, 182 tiles: filter stage
     // 90 us in four sub-batches of 46 tiles, 50 in one)
-    const int tn = tile_n(nu, rows);
     const long tiles = (nu + tn - 1) / tn * ((rows + TM - 2) / (TM - 1));
     return static_cast<int>(std::min<long>(std::max<long>(tiles / (2 * kSms), 1), 4));
 }
@@ -684,10 +689,9 @@ cudaError_t launch_fdk_preweight_split_bf16(const void* proj, int proj_dtype,
 
 cudaError_t launch_fdk_ramp_tcgen05(const __nv_bfloat16* const a_parts[3],
     const __nv_bfloat16* const t_parts[3], int rows, int nu, int ld, const FdkPreweightView* pwv,
-    int nv, float* out, int layout, int ldc, int near_chunks, int* err, cudaStream_t s)
+    int nv, float* out, int layout, int ldc, int tn, int near_chunks, int* err, cudaStream_t s)
 {
     if (rows <= 0) return cudaSuccess;
-    const int tn = tile_n(nu, rows);
     const int nparts = a_parts[2] && t_parts[2] ? 3 : 2;
     CUtensorMap a[3], t[3];
     // A: [rows][ld] K-major, box 64 x 128; T: [nu][ld] K-major, box 64 x TN

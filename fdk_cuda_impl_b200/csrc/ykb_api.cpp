@@ -236,6 +236,7 @@ YKB_API ykb_status ykb_fdk_plan_create_ex(const ykb_cone_view* views, int n_view
                 if (p->tc_parts == 3)
                     t2[at] = __float2bfloat16_rn(static_cast<float>(v - static_cast<double>(__bfloat162float(b1))));
             }
+        p->tc_tile = tc_filter_tile(nu, static_cast<long>(p->batch_capacity) * nv);
         p->tc_near = tc_filter_near_chunks(h, nu);
         if (const char* v = std::getenv("YKB_FDK_FILTER_NEAR"))
             if (std::atoi(v) > 0) p->tc_near = std::atoi(v);
@@ -374,7 +375,7 @@ ykb_status filter_chunk_(ykb_fdk_plan* p, const void* proj, int proj_dtype, int 
         // sub-batches of views: the preweight (memory bound) of sub-batch
         // b + 1 runs on the auxiliary stream under the ramp filter (tensor
         // bound) of sub-batch b
-        const int nsub = std::min(tc_filter_sub_batches(p->nu, static_cast<long>(count) * p->nv), count);
+        const int nsub = std::min(tc_filter_sub_batches(p->tc_tile, p->nu, static_cast<long>(count) * p->nv), count);
         static_assert(ykb_fdk_plan::kFilterSubBatches == 4, "events for every sub-batch");
         if (nsub > 1 && !p->aux_stream) {
             YKB_TRY_CUDA(cudaStreamCreateWithFlags(&p->aux_stream, cudaStreamNonBlocking));
@@ -411,7 +412,7 @@ ykb_status filter_chunk_(ykb_fdk_plan* p, const void* proj, int proj_dtype, int 
             const size_t out_view = layout == kFilteredPairs
                 ? 2 * static_cast<size_t>(ldc) * (p->nv + 1) : static_cast<size_t>(ldc) * p->nv;
             YKB_TRY_CUDA(launch_fdk_ramp_tcgen05(ac, t, (v1 - v0) * p->nv, p->nu, p->lda, pwv + v0,
-                p->nv, dst + v0 * out_view, layout, ldc, p->tc_near, p->err_flag.as<int>(), s));
+                p->nv, dst + v0 * out_view, layout, ldc, p->tc_tile, p->tc_near, p->err_flag.as<int>(), s));
         }
         return YKB_OK;
     }

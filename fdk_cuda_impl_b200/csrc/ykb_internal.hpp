@@ -205,13 +205,17 @@ cudaError_t launch_fdk_preweight_split_bf16(const void* proj, int proj_dtype,
 // the taps' absolute sum.
 cudaError_t launch_fdk_ramp_tcgen05(const __nv_bfloat16* const a_parts[3],
     const __nv_bfloat16* const t_parts[3], int rows, int nu, int ld,
-    const FdkPreweightView* pwv, int nv, float* out, int layout, int ldc, int near_chunks,
+    const FdkPreweightView* pwv, int nv, float* out, int layout, int ldc, int tn, int near_chunks,
     int* err_flag, cudaStream_t s);
 int tc_filter_near_chunks(const std::vector<double>& h, int nu);
 bool tcgen05_filter_supported(int nu);
+// Tile width tn (columns) for calls of `rows` rows.  The 2^-16 products reach whole
+// tiles, so a row's last bits depend on it: a plan keeps one width for all of its
+// calls, however the views are batched
+int tc_filter_tile(int nu, long rows);
 // view sub-batches (1 to 4) in which the preweight of one runs under the filter
 // of the one before
-int tc_filter_sub_batches(int nu, long rows);
+int tc_filter_sub_batches(int tn, int nu, long rows);
 int tc_filter_lda(int nu);
 cudaError_t launch_fdk_backproject(const void* filtered, int dtype,
     const FdkViewCoef* coef, int n_views, int nu, int nv, int ld,
@@ -370,6 +374,7 @@ struct ykb_fdk_plan {
     bool axial = false;
     bool tc_filter = false;
     int tc_parts = 0;            // BF16 parts per operand of the tensor-core filter (2 or 3)
+    int tc_tile = 0;             // its tile width
     int tc_near = 0;             // K chunks each side of a tile that its 2^-16 products cover
     int batch_capacity = 0;      // views the workspace holds
     int ld = 0;                  // row pitch (elements) of the filtered workspace

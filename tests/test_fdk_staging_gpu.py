@@ -103,3 +103,20 @@ def test_column_terms_round_once(oracle, cuda_device, monkeypatch, views, nu, nv
     plan.check()
     plan.close()
     assert K.rel_rmse(rows, oracle.fdk_backproject(table, nu, nv, scan.scan_range, vol, p)) <= bound
+
+
+@pytest.mark.parametrize("nu,nv,views", [(300, 64, 60), (391, 64, 120), (200, 128, 60)])
+def test_filtered_rows_do_not_depend_on_the_batches(oracle, cuda_device, nu, nv, views):
+    # one tile width a plan: a view's rows come out the same to the bit alone, in
+    # batches and with all the others
+    import torch
+    from fdk_cuda_impl_b200.projectors import FdkPlan
+    scan = CircularScan(views, views, 500.0, 1000.0, nu, nv, 0.8, 0.8)
+    plan = FdkPlan(scan.views(), nu, nv, scan.scan_range, VolumeGrid.cube(16, 1.0), RampFilter())
+    p = torch.from_numpy(oracle.uniform((views, nv, nu), 0.5, 1.5, 4)).cuda()
+    whole = plan.filter(p)
+    for n in (1, 7):
+        parts = [plan.filter(p[k:k + n].contiguous(), view_offset=k) for k in range(0, views, n)]
+        assert torch.equal(torch.cat(parts), whole)
+    plan.check()
+    plan.close()
