@@ -218,7 +218,7 @@ bool small_volume(const VolumeGrid& g)
 // crossings of flat rays keep their place.
 // Bound: instruction issue (22 a segment and ray, 63 % in the projector, 71 % in
 // the backprojector, whose reductions keep L2 half busy).  256^3 x 120 x 384^2:
-// 5.2 and 6.7 ms, before 7.3 and 11.9; error against FP64 7.5e-7, before 7.7e-7
+// 5.2 and 6.0 ms, before 7.3 and 11.9; error against FP64 7.5e-7, before 7.7e-7
 // (8.1e-7 while the face distances were rounded once per axis).
 // ---------------------------------------------------------------------------
 constexpr int kLineCols = 4;
@@ -361,9 +361,10 @@ __device__ __forceinline__ LineStep line_step(LineRay& r, float s1)
 template <bool FORWARD>
 __global__ void __launch_bounds__(kLineRows + 32, 6) siddon_lines_kernel(const float* __restrict__ in,
     const ykb_cone_view* __restrict__ views, int view0, int nu, int nv, const __grid_constant__ VolumeGrid g,
-    int nzp, float* __restrict__ out, long half, int accumulate)
+    int nzp, float* __restrict__ out, float* __restrict__ odd, int accumulate)
 {
-    if constexpr (!FORWARD) out += ((view0 + blockIdx.z) & 1) * half;
+    if constexpr (!FORWARD)
+        if ((view0 + blockIdx.z) & 1) out = odd;
     __shared__ float2 segments[2][kLineSegments][kLineCols];
     __shared__ int more[2];
     const int tid = threadIdx.x, rows = blockDim.x - 32;
@@ -439,10 +440,10 @@ __global__ void __launch_bounds__(kLineRows + 32, 6) siddon_lines_kernel(const f
     }
 }
 
-// vol[z][y][x] (+)= both halves of vt[x][y][z] (rows of nzp, kLinePad rows around
+// vol[z][y][x] (+)= vt[x][y][z] + odd[x][y][z] (rows of nzp, kLinePad rows around
 // x and y)
-__global__ void __launch_bounds__(256) untranspose_xyz_kernel(const float* __restrict__ vt, long half,
-    int nx, int ny, int nz, int nzp, float* __restrict__ vol, int accumulate)
+__global__ void __launch_bounds__(256) untranspose_xyz_kernel(const float* __restrict__ vt,
+    const float* __restrict__ odd, int nx, int ny, int nz, int nzp, float* __restrict__ vol, int accumulate)
 {
     __shared__ float tile[32][33];
     const int y = blockIdx.z, x0 = blockIdx.x * 32, z0 = blockIdx.y * 32;
@@ -451,7 +452,7 @@ __global__ void __launch_bounds__(256) untranspose_xyz_kernel(const float* __res
         if (x < nx && z < nz)
         {
             const long at = (static_cast<long>(x + kLinePad) * (ny + 2 * kLinePad) + y + kLinePad) * nzp + z;
-            tile[r][threadIdx.x] = vt[at] + vt[half + at];
+            tile[r][threadIdx.x] = vt[at] + odd[at];
         }
     }
     __syncthreads();
@@ -500,28 +501,28 @@ cudaError_t launch_siddon_fp_lines(const float* vol, float* vt, const ykb_cone_v
         int threads = 0;
         const dim3 grid = line_grid(nu, nv, min(n_views - done, 65535), threads);
         siddon_lines_kernel<true><<<grid, threads, 0, s>>>(vt, views, done, nu, nv, g,
-            joseph_line_pitch(g.nz), proj, 0, accumulate);
+            joseph_line_pitch(g.nz), proj, nullptr, accumulate);
         e = cudaGetLastError();
     }
     return e;
 }
 
-cudaError_t launch_siddon_bp_lines(const float* proj, float* vt, const ykb_cone_view* views, int n_views,
-    int nu, int nv, const VolumeGrid& g, float* vol, int accumulate, cudaStream_t s)
+cudaError_t launch_siddon_bp_lines(const float* proj, float* vt, float* odd, const ykb_cone_view* views,
+    int n_views, int nu, int nv, const VolumeGrid& g, float* vol, int accumulate, cudaStream_t s)
 {
     const int nzp = joseph_line_pitch(g.nz);
     const size_t elems = static_cast<size_t>(g.nx + 2 * kLinePad) * (g.ny + 2 * kLinePad) * nzp;
-    cudaError_t e = cudaMemsetAsync(vt, 0, 2 * sizeof(float) * elems, s);
+    cudaError_t e = cudaMemsetAsync(vt, 0, sizeof(float) * elems, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(odd, 0, sizeof(float) * elems, s);
     for (int done = 0; e == cudaSuccess && done < n_views; done += 65535) {
         int threads = 0;
         const dim3 grid = line_grid(nu, nv, min(n_views - done, 65535), threads);
-        siddon_lines_kernel<false><<<grid, threads, 0, s>>>(proj, views, done, nu, nv, g, nzp, vt,
-            static_cast<long>(elems), 0);
+        siddon_lines_kernel<false><<<grid, threads, 0, s>>>(proj, views, done, nu, nv, g, nzp, vt, odd, 0);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) return e;
-    untranspose_xyz_kernel<<<dim3((g.nx + 31) / 32, (g.nz + 31) / 32, g.ny), dim3(32, 8), 0, s>>>(vt,
-        static_cast<long>(elems), g.nx, g.ny, g.nz, nzp, vol, accumulate);
+    untranspose_xyz_kernel<<<dim3((g.nx + 31) / 32, (g.nz + 31) / 32, g.ny), dim3(32, 8), 0, s>>>(vt, odd,
+        g.nx, g.ny, g.nz, nzp, vol, accumulate);
     return cudaGetLastError();
 }
 

@@ -894,7 +894,7 @@ YKB_API size_t ykb_joseph_workspace_bytes(const ykb_joseph_plan* p)
     if (!p) return 0;
     return p->views.bytes + p->view_proj.bytes + p->rays.bytes + p->lens.bytes +
         p->weighted.bytes + p->cols.bytes + p->heights.bytes + p->vt.bytes + p->slab_x.bytes + p->slab_y.bytes +
-        p->world_views.bytes +
+        p->world_views.bytes + p->siddon_odd.bytes +
         p->fdk_coef.bytes +
         p->pseudo_coef.bytes + p->pairs.bytes + p->err_flag.bytes;
 }
@@ -1006,14 +1006,14 @@ ykb_status pseudo_bp(ykb_joseph_plan* p, const float* d_proj, float* d_volume, i
     return YKB_OK;
 }
 
-// The views and, for the pair by detector columns, its volume copy, in one
+// The views and, for the pair by detector columns, its first volume copy, in one
 // allocation; without room for the copy the rays are walked one by one.
 ykb_status prepare_siddon(ykb_joseph_plan* p, const VolumeGrid& g, cudaStream_t s)
 {
     const size_t views = sizeof(ykb_cone_view) * p->cone_views.size();
     const size_t at = (views + 255) / 256 * 256;
     const size_t copy = siddon_lines_apply(p->cone_views.data(), p->n_views, p->nv, g)
-        ? 2 * sizeof(float) * joseph_line_elems(p->volume) : 0;
+        ? sizeof(float) * joseph_line_elems(p->volume) : 0;
     bool lines = copy > 0;
     cudaError_t e = cudaSuccess;
     if (lines && !p->siddon_done) e = cudaEventCreateWithFlags(&p->siddon_done, cudaEventDisableTiming);
@@ -1047,7 +1047,13 @@ ykb_status siddon(ykb_joseph_plan* p, bool forward, const float* d_in, float* d_
     // orders then: a captured call takes the walk, which shares no workspace
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     YKB_TRY_CUDA(cudaStreamIsCapturing(s, &capture));
-    if (!p->siddon_vt || capture != cudaStreamCaptureStatusNone) {
+    bool lines = p->siddon_vt && capture == cudaStreamCaptureStatusNone;
+    if (lines && !forward && !p->siddon_odd.ptr &&
+        p->siddon_odd.alloc(sizeof(float) * joseph_line_elems(p->volume)) != cudaSuccess) {
+        cudaGetLastError();
+        lines = false;
+    }
+    if (!lines) {
         if (forward)
             YKB_TRY_CUDA(launch_siddon_fp(d_in, v, p->n_views, p->nu, p->nv, g, d_out, accumulate, s));
         else
@@ -1059,7 +1065,8 @@ ykb_status siddon(ykb_joseph_plan* p, bool forward, const float* d_in, float* d_
     if (forward)
         YKB_TRY_CUDA(launch_siddon_fp_lines(d_in, vt, v, p->n_views, p->nu, p->nv, g, d_out, accumulate, s));
     else
-        YKB_TRY_CUDA(launch_siddon_bp_lines(d_in, vt, v, p->n_views, p->nu, p->nv, g, d_out, accumulate, s));
+        YKB_TRY_CUDA(launch_siddon_bp_lines(d_in, vt, p->siddon_odd.as<float>(), v, p->n_views, p->nu, p->nv, g,
+            d_out, accumulate, s));
     YKB_TRY_CUDA(cudaEventRecord(p->siddon_done, s));
     return YKB_OK;
 }

@@ -335,13 +335,13 @@ cudaError_t launch_siddon_bp(const float* proj, const ykb_cone_view* views, int 
     int nv, const VolumeGrid& g, float* vol, int accumulate, cudaStream_t s);
 // The same pair for axial-column scans by detector columns, over the volume copy
 // of joseph_line_elems floats (see launch_joseph_line_volume); the backprojector
-// sums even and odd views in a copy each: half the additions to a voxel, to sums
-// half as large, so half their rounding
+// sums even and odd views in a copy each (vt, odd): half the additions to a voxel,
+// to sums half as large, so half their rounding
 bool siddon_lines_apply(const ykb_cone_view* views, int n_views, int nv, const VolumeGrid& g);
 cudaError_t launch_siddon_fp_lines(const float* vol, float* vt, const ykb_cone_view* views, int n_views,
     int nu, int nv, const VolumeGrid& g, float* proj, int accumulate, cudaStream_t s);
-cudaError_t launch_siddon_bp_lines(const float* proj, float* vt, const ykb_cone_view* views, int n_views,
-    int nu, int nv, const VolumeGrid& g, float* vol, int accumulate, cudaStream_t s);
+cudaError_t launch_siddon_bp_lines(const float* proj, float* vt, float* odd, const ykb_cone_view* views,
+    int n_views, int nu, int nv, const VolumeGrid& g, float* vol, int accumulate, cudaStream_t s);
 // (a1, e1) of every detector column from its first row into cols[n][nu];
 // flag[0] = 1 when any ray of a column differs (the line backprojector
 // then does not apply)
@@ -458,9 +458,11 @@ struct ykb_joseph_plan {
     ykb::JosephFpLines fp_lines;       // forward projection by lines (column_bp scans)
     ykb::DeviceBuffer vt;              // its volume copy [x][y][z]
     // Siddon, set up on first use: the views, and for untilted scans a volume copy
-    // behind them.  Calls on different streams take turns on the copy
+    // behind them; the first backprojection adds the copy that sums the odd views.
+    // Calls on different streams take turns on the copies
     ykb::DeviceBuffer world_views;     // ykb_cone_view[n], then the copy
     float* siddon_vt = nullptr;        // (null: the rays are walked one by one)
+    ykb::DeviceBuffer siddon_odd;      // (empty: the backprojector walks them so)
     cudaEvent_t siddon_done = nullptr; // the last call's work on the copy
     std::mutex siddon_mutex;
     ~ykb_joseph_plan() { if (siddon_done) cudaEventDestroy(siddon_done); }

@@ -316,9 +316,15 @@ typedef enum ykb_task {
  *     exact intersection lengths of the source-to-pixel-centre ray with each
  *     voxel (fp_siddon_launch, src/FlatFpBp/FP/kernels/YkFPSiddonKernel.cu:
  *     19-129,283-316; bp_siddon_launch, src/FlatFpBp/BP/kernels/
- *     YkBPSiddonKernel.cu:31-160).  The backprojector is the exact transpose
- *     of the projector; it sums with global atomics, so its last bits vary
- *     between runs.
+ *     YkBPSiddonKernel.cu:31-160).  The backprojector is the transpose of the
+ *     projector, up to FP32 rounding; it sums with global atomics, so its last
+ *     bits vary between runs.  The plan's first Siddon call copies the views
+ *     (synchronising the stream).  Untilted scans are projected by detector
+ *     columns: their first projection allocates one volume copy, kept with
+ *     the plan, and their first backprojection a second one; without room for
+ *     it, and in a call under stream capture, the rays are walked one by one,
+ *     which is slower and rounds differently.  Calls on several streams share
+ *     the copies and take turns on the GPU.
  *   YKB_TASK_BP_FDK_PSEUDO_MATCHED: voxel-driven bilinear backprojection
  *     with the weight L^3 / (|P - S|^2 SDD_plane) x voxel volume / pixel
  *     area (fdk_pseudo_matched_bp_launch, src/FlatFpBp/BP/kernels/

@@ -12,7 +12,8 @@ namespace {
 
 size_t g_capacity = ~size_t(0), g_used = 0;
 std::map<void*, size_t> g_blocks;
-int g_failures = 0;
+int g_failures = 0, g_lines = 0, g_walks = 0;
+bool g_capturing = false;
 
 void expect(bool ok, const char* what)
 {
@@ -58,6 +59,19 @@ cudaError_t cudaMemsetAsync(void*, int, size_t, cudaStream_t) { return cudaSucce
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = nullptr; return cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* status)
+{
+    *status = g_capturing ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
+    return cudaSuccess;
+}
+cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned)
+{
+    *e = reinterpret_cast<cudaEvent_t>(1);
+    return cudaSuccess;
+}
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 }
 
 namespace ykb {
@@ -73,6 +87,31 @@ cudaError_t launch_joseph_ray_heights(const float4*, long, float2*, cudaStream_t
 JosephFpLines joseph_fp_lines_shape(const std::vector<JosephView>&, int) { return {128, 144}; }
 bool joseph_bp_runs(const std::vector<JosephView>&, int) { return true; }
 int joseph_bp_splits(const ykb_volume&, int) { return 4; }
+bool siddon_lines_apply(const ykb_cone_view*, int, int, const VolumeGrid&) { return true; }
+cudaError_t launch_siddon_fp(const float*, const ykb_cone_view*, int, int, int, const VolumeGrid&, float*, int,
+    cudaStream_t)
+{
+    ++g_walks;
+    return cudaSuccess;
+}
+cudaError_t launch_siddon_bp(const float* in, const ykb_cone_view* v, int n, int nu, int nv, const VolumeGrid& g,
+    float* out, int accumulate, cudaStream_t s)
+{
+    return launch_siddon_fp(in, v, n, nu, nv, g, out, accumulate, s);
+}
+cudaError_t launch_siddon_fp_lines(const float*, float* vt, const ykb_cone_view*, int, int, int,
+    const VolumeGrid&, float*, int, cudaStream_t)
+{
+    expect(vt != nullptr, "the projector's copy");
+    ++g_lines;
+    return cudaSuccess;
+}
+cudaError_t launch_siddon_bp_lines(const float* in, float* vt, float* odd, const ykb_cone_view* v, int n,
+    int nu, int nv, const VolumeGrid& g, float* out, int accumulate, cudaStream_t s)
+{
+    expect(odd != nullptr && odd != vt, "the backprojector's second copy");
+    return launch_siddon_fp_lines(in, vt, v, n, nu, nv, g, out, accumulate, s);
+}
 } // namespace ykb
 
 using namespace ykb;
@@ -164,6 +203,40 @@ void optional_buffers()
     expect(g_used == 0 && g_blocks.empty(), "everything given back");
 }
 
+// The projector holds one volume copy, the backprojector two; without room for
+// them, and under capture, the rays are walked one by one
+void siddon_copies()
+{
+    const Scan scan(24, 40, 36, 64, 60, 48);
+    const size_t copy = sizeof(float) * joseph_line_elems(scan.volume);
+    float in = 0.f, out = 0.f;
+    // room for: nothing of it, the views, one copy, both
+    for (int room = 0; room < 4; ++room) {
+        ykb_joseph_plan* p = scan.joseph();
+        if (!p) return;
+        const size_t before = g_used, views = 24 * sizeof(ykb_cone_view);
+        const size_t one = (views + 255) / 256 * 256 + copy;
+        g_capacity = before + (room == 0 ? views - 1 : room == 1 ? one - 1 : room == 2 ? one + copy - 1 : one + copy);
+        g_lines = g_walks = 0;
+        ykb_status st = ykb_operator_apply(p, YKB_TASK_FP_SIDDON, &in, &out, 0, nullptr);
+        expect((st == YKB_OK) == (room > 0), "views are needed");
+        expect(g_lines == (room > 1) && g_walks == (room == 1), "the projector's kernel");
+        expect(g_used - before == (room == 0 ? 0 : room == 1 ? views : one), "one copy for the projector");
+        st = ykb_operator_apply(p, YKB_TASK_BP_SIDDON_RAY_DRIVEN, &in, &out, 0, nullptr);
+        expect((st == YKB_OK) == (room > 0), "views are needed");
+        expect(g_lines == (room > 1) + (room > 2) && g_walks == (room == 1 ? 2 : room == 2), "the backprojector's");
+        expect(g_used - before == (room == 3 ? one + copy : room == 2 ? one : room == 1 ? views : 0), "both copies");
+        if (room == 3) {
+            g_capturing = true;
+            ykb_operator_apply(p, YKB_TASK_FP_SIDDON, &in, &out, 0, nullptr);
+            g_capturing = false;
+            expect(g_walks == 1 && g_lines == 2, "captured calls walk");
+        }
+        ykb_joseph_plan_destroy(p);
+        expect(g_used == 0, "everything given back");
+    }
+}
+
 } // namespace
 
 int main(int argc, char** argv)
@@ -171,6 +244,7 @@ int main(int argc, char** argv)
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "line_volume") line_volume();
     else if (what == "optional_buffers") optional_buffers();
+    else if (what == "siddon_copies") siddon_copies();
     else return 2;
     return g_failures ? 1 : 0;
 }

@@ -20,7 +20,7 @@ def plan_bin(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("what", ["line_volume", "optional_buffers"])
+@pytest.mark.parametrize("what", ["line_volume", "optional_buffers", "siddon_copies"])
 def test_plan_memory(plan_bin, what):
     res = subprocess.run([plan_bin, what], capture_output=True, text=True, timeout=60)
     assert res.returncode == 0, res.stderr
