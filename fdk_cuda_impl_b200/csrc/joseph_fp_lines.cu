@@ -241,8 +241,9 @@ __global__ void __launch_bounds__(kMaxRows, 2) joseph_fp_lines_kernel(const floa
         const int zb = zlo & ~3;  // 16-byte loads of the volume rows
         bool some = zhi >= 0 && zlo < nz;
         if (some && zhi - zb >= W) {
-            // wider than the host's bound (no case is known): straight from the
-            // volume, so that no shared access leaves its line
+            // wider than the host's bound (no scan is known; a test narrows the
+            // window): straight from the volume, so that no shared access leaves
+            // its line
             some = false;
             sample_volume(vt, st_1, nz, tables + (b % kTables) * 32, a2, e2, c0, acc);
         }

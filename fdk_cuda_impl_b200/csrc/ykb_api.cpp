@@ -832,6 +832,10 @@ YKB_API ykb_status ykb_joseph_plan_create(const ykb_cone_view* views, int n_view
         if (!p->column_bp) p->cols.reset();
         if (p->column_bp) {
             if (joseph_line_volume_fits(*volume)) p->fp_lines = joseph_fp_lines_shape(p->host_views, nv);
+            // YKB_JOSEPH_FP_WINDOW=<floats> sets the lines' window (tests of the
+            // samples taken past one that is too narrow)
+            if (const char* env = std::getenv("YKB_JOSEPH_FP_WINDOW"))
+                if (p->fp_lines.rows > 0 && std::atoi(env) > 0) p->fp_lines.window = std::atoi(env);
             // (32-bit byte offsets of a view's ray records)
             p->bp_runs = static_cast<long>(nu) * nv < (1L << 27) && joseph_bp_runs(p->host_views, nv);
         }

@@ -21,8 +21,9 @@ CASES = [
     (10, 65, 33, 1.1, 1.3, (37, 41, 30), (0.8, 0.9, 1.1), False),
     (8, 40, 97, 1.6, 0.2, (24, 24, 40), (1.0, 1.0, 1.0), True),     # rows a tenth of a voxel apart
     (8, 40, 24, 1.6, 9.0, (24, 24, 120), (1.0, 1.0, 1.0), False),   # rows 4.5 voxels apart
-    (8, 24, 130, 1.6, 14.0, (20, 20, 900), (1.0, 1.0, 1.0), False),  # and too far for the lines' window
+    (8, 24, 130, 1.6, 14.0, (20, 20, 900), (1.0, 1.0, 1.0), False),  # 7 voxels: the 304-float window
     (6, 30, 500, 1.6, 1.6, (40, 36, 420), (1.0, 1.0, 1.0), False),
+    (8, 24, 130, 1.6, 26.0, (20, 20, 1700), (1.0, 1.0, 1.0), False),  # 13: no window, the slab projector
 ]
 
 
@@ -106,3 +107,54 @@ def test_infinite_rays_stay_infinite(cuda_device, runs):
         assert not torch.isnan(inf).any()
         assert torch.equal(one != 0, torch.isinf(inf))
     plan.close()
+
+
+@pytest.mark.parametrize("case", [CASES[i] for i in (2, 5, 6, 7)])
+def test_samples_past_a_narrow_window(oracle, cuda_device, monkeypatch, case):
+    # YKB_JOSEPH_FP_WINDOW=64 leaves CTAs of these cases (windows of 96 to 304)
+    # one too narrow for their rays; their samples then come from the volume, the
+    # same to the bit
+    import torch
+    from fdk_cuda_impl_b200.projectors import JosephPlan
+    views, nu, nv, pu, pv, n, vox, flipped = case
+    scan = CircularScan(views, views, 500.0, 1000.0, nu, nv, pu, pv, start_angle_rad=0.05)
+    grid = VolumeGrid(*n, vox, (0.4, -0.7, 0.2))
+    x = torch.from_numpy(oracle.uniform(grid.shape, 0.0, 1.0, 3)).cuda()
+    plan = JosephPlan(scan.views(), nu, nv, grid)
+    expected = plan.forward(x)
+    plan.close()
+    monkeypatch.setenv("YKB_JOSEPH_FP_WINDOW", "64")
+    narrow = JosephPlan(scan.views(), nu, nv, grid)
+    assert torch.equal(narrow.forward(x), expected)
+    narrow.close()
+
+
+def test_plan_without_room_for_its_table(oracle, cuda_device):
+    # with the GPU's memory taken but for what the plan cannot do without, the
+    # rays' heights are read from the ray records: the same results to the bit
+    import torch
+    from fdk_cuda_impl_b200.projectors import JosephPlan
+    views, det = 80, 256
+    scan = CircularScan(views, views, 500.0, 1000.0, det, det, 0.9, 0.9, start_angle_rad=0.05)
+    grid = VolumeGrid(128, 128, 120, (1.0, 1.0, 1.0))
+    x = torch.from_numpy(oracle.uniform(grid.shape, 0.0, 1.0, 3)).cuda()
+    y = torch.from_numpy(oracle.normal((views, det, det), 7)).cuda()
+    plan = JosephPlan(scan.views(), det, det, grid)
+    full = plan.workspace_bytes()
+    a, b = plan.forward(x), plan.adjoint(y)
+    a2, b2 = torch.empty_like(a), torch.empty_like(b)
+    plan.close()
+    table = 8 * views * det * det
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    taken = torch.empty(free - (full - table // 2), dtype=torch.uint8, device="cuda")
+    try:
+        plan = JosephPlan(scan.views(), det, det, grid)
+        assert plan.workspace_bytes() == full - table
+        assert torch.equal(plan.forward(x, a2), a)
+        assert torch.equal(plan.adjoint(y, b2), b)
+        plan.close()
+    finally:
+        del taken
+        torch.cuda.empty_cache()
