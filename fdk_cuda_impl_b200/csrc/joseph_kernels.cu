@@ -367,6 +367,8 @@ __device__ __forceinline__ void footprint_box_range(const ViewProj& m, const Jos
         const float w = fmaf(m.m[8], px, fmaf(m.m[9], py, fmaf(m.m[10], pz, m.m[11])));
         // one ulp of the reciprocal moves a corner by less than the margin below
         // column 400000
+        // (correctly rounded: the 256^3 gradient step 31.0 ms instead of 30.5, the
+        // tilted one 5.60 instead of 5.45, the same results)
         float rw;
         asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rw) : "f"(w));
         const float u = fmaf(m.m[0], px, fmaf(m.m[1], py, fmaf(m.m[2], pz, m.m[3]))) * rw;

@@ -343,8 +343,8 @@ def test_fdk_execute_host_matches_device(oracle, cuda_device, pinned, precision)
 @pytest.mark.parametrize("nz", [48, 100])
 def test_fdk_execute_host_out(oracle, cuda_device, nz):
     # host projections in, host volume out: the last batch runs in z slabs of
-    # whole 48-slice z tiles whose downloads overlap the next slab (nz = 48:
-    # one slab; nz = 100: slabs of 48, 48 and 4 slices)
+    # whole 64-slice z tiles whose downloads overlap the next slab (nz = 48:
+    # one slab; nz = 100: slabs of 64 and 36 slices)
     import torch
     from fdk_cuda_impl_b200.geometry import VolumeGrid
     from fdk_cuda_impl_b200.projectors import FdkPlan
@@ -430,10 +430,10 @@ def test_fdk_parker_modes(oracle, cuda_device):
 
 @pytest.mark.parametrize("withheld", [0, 5, 59])
 def test_pipeline_wait_timeout_is_reported_and_the_plan_recovers(oracle, cuda_device, withheld):
-    # The TMA backprojection bounds every pipeline wait.  The test hook makes
-    # the copy producer withhold one view and shortens the waits to 1 ms:
-    # every CTA's consumers give up on that view, its producer gives up on
-    # the stage they never release, drains the copies it issued and ends.
+    # The TMA backprojection bounds every pipeline wait.  The test hook
+    # withholds the copy of one view and shortens the waits to 1 ms: every
+    # CTA's warps give up on that view, the CTA drains the copies that it
+    # issued and ends.
     # ykb_fdk_check reports the timeout; afterwards the same plan, with the
     # default limit restored, reproduces its earlier result bit for bit.
     import torch

@@ -11,6 +11,13 @@ from tests import cases as K
 
 pytestmark = pytest.mark.gpu
 
+# A length's two ends are FP32 distances below 128 mm from the middle of the ray:
+# rms 2.2e-6 mm each, 3.1e-6 of a voxel a millimetre wide, which is the relative
+# error of a backprojection of white noise.  A projection averages it over its
+# segments (16 and more, of values that differ by a half), beside its FP32 sum
+BP_TOL = 3.1e-6
+FP_TOL = 6e-7
+
 CASES = [
     # views, nu, nv, pixel u, pixel v, (nx, ny, nz), voxel, flipped
     (9, 1, 1, 2.0, 2.0, (5, 4, 1), (1.0, 1.0, 1.0), False),
@@ -39,12 +46,12 @@ def test_siddon_pair_matches_oracle(oracle, cuda_device, case):
     plan = JosephPlan(table, nu, nv, grid)
     fp, bp = plan.forward_siddon(xd), plan.backproject_siddon(yd)
     ref_fp, ref_bp = oracle.siddon_fp(table, nu, nv, vol, x), oracle.siddon_bp(table, nu, nv, vol, y)
-    assert K.rel_rmse(fp.cpu().numpy(), ref_fp) <= 1e-5
-    assert K.rel_rmse(bp.cpu().numpy(), ref_bp) <= 1e-5
+    assert K.rel_rmse(fp.cpu().numpy(), ref_fp) <= FP_TOL
+    assert K.rel_rmse(bp.cpu().numpy(), ref_bp) <= BP_TOL
     twice = plan.forward_siddon(xd, fp.clone(), accumulate=True)
-    assert K.rel_rmse(twice.cpu().numpy(), 2 * ref_fp) <= 1e-5
+    assert K.rel_rmse(twice.cpu().numpy(), 2 * ref_fp) <= FP_TOL
     both = plan.backproject_siddon(yd, bp.clone(), accumulate=True)
-    assert K.rel_rmse(both.cpu().numpy(), 2 * ref_bp) <= 1e-5
+    assert K.rel_rmse(both.cpu().numpy(), 2 * ref_bp) <= BP_TOL
     # two streams in turn
     torch.cuda.synchronize()
     streams = [torch.cuda.Stream(), torch.cuda.Stream()]
@@ -54,15 +61,15 @@ def test_siddon_pair_matches_oracle(oracle, cuda_device, case):
             out.append(plan.forward_siddon(xd) if i % 3 else plan.backproject_siddon(yd))
     torch.cuda.synchronize()
     for i, o in enumerate(out):
-        assert K.rel_rmse(o.cpu().numpy(), ref_fp if i % 3 else ref_bp) <= 1e-5
+        assert K.rel_rmse(o.cpu().numpy(), ref_fp if i % 3 else ref_bp) <= BP_TOL
     # a captured call
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
         gp, gb = plan.forward_siddon(xd), plan.backproject_siddon(yd)
     graph.replay()
     torch.cuda.synchronize()
-    assert K.rel_rmse(gp.cpu().numpy(), ref_fp) <= 1e-5
-    assert K.rel_rmse(gb.cpu().numpy(), ref_bp) <= 1e-5
+    assert K.rel_rmse(gp.cpu().numpy(), ref_fp) <= FP_TOL
+    assert K.rel_rmse(gb.cpu().numpy(), ref_bp) <= BP_TOL
     # a voxel that no ray of a missing column reads does not leak into it
     if n[0] > 20:
         bad = xd.clone()
