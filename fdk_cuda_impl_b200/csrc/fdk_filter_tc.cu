@@ -614,7 +614,7 @@ cudaError_t launch_tn(const CUtensorMap* a, const CUtensorMap* t, int nseg, long
 
 namespace {
 
-constexpr int kSms = 148;
+constexpr int kSms = 148;  // for the choice of a width only: the launch asks the device
 
 // Tile width that filters `rows` rows of nu columns soonest.  The operand feed
 // bounds the tiles (48 KB a K step at 256 columns, 24 at 64, from L2), and every

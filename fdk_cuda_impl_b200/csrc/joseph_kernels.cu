@@ -787,12 +787,13 @@ __global__ void __launch_bounds__(kLineThreads, 3) joseph_bp_lines_kernel(
 //   * the last warp, which the lines rarely reach, prepares the next view's
 //     boxes, and every thread has its next line's first rays in flight while it
 //     sums its column: two barriers a view.
-// Bound: instruction issue and the shared-memory data path together (59 and 62 %;
-// three wavefronts a request in the column sums), with 24 warps an SM.  256^3 x
-// 360 x 384^2: 20.2 ms, before 24.9; scalar instead of packed sums of the two
-// slices: 20.5; the runs alone, without the last two points: 25.2; (a2, e2) from
-// the 16-byte ray records instead of a table of their own: 22.2 against 21.1; two
-// sets of rays in turn instead of a copy of the set in flight: 22.1 (spills).
+// Bound: the latency of the two phases between their barriers, with 24 warps an SM;
+// nothing is saturated (issue 58 %, L1 data path 61 % of its wavefronts, three a
+// request in the column sums).  256^3 x 360 x 384^2: 20.2 ms, before 24.9; scalar
+// instead of packed sums of the two slices: 20.5; the runs alone, without the last
+// two points: 25.2; (a2, e2) from the 16-byte ray records instead of a table of
+// their own: 22.2 against 21.1; two sets of rays in turn instead of a copy of the
+// set in flight: 22.1 (spills).
 // ---------------------------------------------------------------------------
 constexpr int kRunGroup = 4;  // rays of a line loaded together
 

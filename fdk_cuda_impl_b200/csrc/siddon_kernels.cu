@@ -210,14 +210,15 @@ bool small_volume(const VolumeGrid& g)
 // in one voxel or crosses one z face (checked by the host: it climbs less than a
 // voxel over the longest segment).  A CTA owns kLineCols detector columns and up
 // to 128 rows; an extra warp walks the columns a batch of segments ahead, a lane
-// a column.  Against the walk above: about 20 instructions per in-plane segment
-// for 35 per voxel crossed, all lanes alive to the end, and the volume copy
-// [x][y][z] makes a warp's accesses a run of neighbouring z.
+// a column.  Against the walk above: 22 instructions per in-plane segment in the
+// projector and 29 in the backprojector for 35 per voxel crossed, all lanes alive
+// to the end, and the volume copy [x][y][z] makes a warp's accesses a run of
+// neighbouring z.
 // Distances are measured from the middle of the ray's way through the volume and
 // heights from the voxel it is in there, so that both stay small and face
 // crossings of flat rays keep their place.
-// Bound: instruction issue (22 a segment and ray, 63 % in the projector, 71 % in
-// the backprojector, whose reductions keep L2 half busy).  256^3 x 120 x 384^2:
+// Bound: issue and the latency of its gathers in the projector (66 % issue), issue
+// in the backprojector (76 %), whose reductions keep L2 half busy.  256^3 x 120 x 384^2:
 // 5.2 and 6.0 ms, before 7.3 and 11.9; error against FP64 7.5e-7, before 7.7e-7
 // (8.1e-7 while the face distances were rounded once per axis).
 // ---------------------------------------------------------------------------

@@ -476,9 +476,9 @@ ykb_status backproject_chunk(ykb_fdk_plan* p, const void* filtered, int layout, 
 // views: the kernels wait only for the first, short copy, and each later
 // copy (a view copies in about half the time its kernels take) completes
 // while the previous batch is processed; a remainder of between one and two
-// batches runs as two halves.  Few batches matter: each backprojection
-// launch costs about 0.8 ms beyond its views (512^3 x 720: 64.6 ms in one
-// launch, 75.7 ms in seven).  With h_volume, the last batch is
+// batches runs as two halves.  Few batches are better: each costs about
+// 0.3 ms beyond its views (512^3 x 720 from device memory: 56.6 ms in one
+// batch, 58.3 ms in seven).  With h_volume, the last batch is
 // backprojected in z slabs of whole z tiles, about a quarter of the volume
 // each (two 64-slice layers of 512 CTAs at 512^3 fill whole waves of 148
 // SMs, where one layer leaves half a wave idle), and each finished slab is
